@@ -112,23 +112,21 @@ void glsfft::tc_tables_destroy(TcTables *t) {
     *t = TcTables{};
 }
 
-// Per-pass tables (see tw_offset), for every radix R and every length
-// R <= L <= kTwRadixSpan / 2: row k < L/R of table (R, L) holds
+// Per-pass tables (see tw_offset, tw_entry), for every radix R and every
+// length R <= L <= kTwRadixSpan / 2: position k < L/R of table (R, L) holds
 // w^r = e^{-2 pi i k r / L} for 1 <= r < R/2 in slot r and w^(R/2) in slot 0
 // (the line engine derives w^(R/2+r) = w^(R/2) w^r); for R = 2 slot 0 holds w^1.
 void glsfft::make_twiddle_host(float2 *dst) {
     for (int i = 0; i < kTwEntries; i++) dst[i] = make_float2(0.f, 0.f);
     for (int radix = 2; radix <= 16; radix <<= 1)
-        for (int l = radix; l <= kTwRadixSpan / 2; l <<= 1)
+        for (int l = radix; l <= kTwRadixSpan / 2; l <<= 1) {
+            float2 *table = dst + tw_offset(radix, l);
             for (int k = 0; k < l / radix; k++) {
-                float2 *row = dst + tw_offset(radix, l) + k * radix;
-                if (radix == 2) {
-                    row[0] = twiddle(k, l);
-                    continue;
-                }
-                row[0] = twiddle((long long)k * (radix / 2), l);
-                for (int r = 1; r < radix / 2; r++) row[r] = twiddle((long long)k * r, l);
+                table[tw_entry(radix, l, k, 0)] = twiddle((long long)k * (radix / 2), l);
+                for (int r = 1; r < radix / 2; r++)
+                    table[tw_entry(radix, l, k, r)] = twiddle((long long)k * r, l);
             }
+        }
 }
 
 // ---------------------------------------------------------------- helpers

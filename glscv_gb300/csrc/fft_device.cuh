@@ -194,29 +194,23 @@ struct SyncCompute256 {
 };
 
 // ------------------------------------------------------ twiddle sources
-// Row k of the table of a pass with radix R and span L = Ns*R: w^(R/2) in
-// w[0] (R > 2) and w^1..w^(R/2-1) in w[1..], w = e^{-2 pi i k / L}; for
-// R = 2, w[0] = w^1.  From the global tables (tw_offset layout):
+// The pair of twiddles (2h, 2h+1) of butterfly position k of a pass with
+// radix R and span L = Ns*R: slot r holds w^r, slot 0 w^(R/2) (R > 2),
+// w = e^{-2 pi i k / L}; for R = 2 the one entry is w^1.  From the global
+// tables (tw_offset, tw_entry):
 template <int N, int MB, int P_, int R, int L>
-__device__ __forceinline__ void tw_row(const float2 *__restrict__ tw, int k, float2 (&w)[R / 2]) {
-    const float2 *wt = tw + tw_offset(R, L) + k * R;
-    if constexpr (R == 2) {
-        w[0] = __ldg(wt);
-    } else {
-        const float4 *w4 = reinterpret_cast<const float4 *>(wt);
-#pragma unroll
-        for (int h = 0; h < R / 4; h++) {
-            const float4 q = __ldg(w4 + h);
-            w[2 * h] = make_float2(q.x, q.y);
-            w[2 * h + 1] = make_float2(q.z, q.w);
-        }
-    }
+__device__ __forceinline__ float4 tw_pair(const float2 *__restrict__ tw, int k, int h) {
+    static_assert(R >= 4, "pairs need radix >= 4");
+    return __ldg(reinterpret_cast<const float4 *>(tw + tw_offset(R, L)) + h * (L / R) + k);
+}
+template <int N, int MB, int P_, int L>
+__device__ __forceinline__ float2 tw_single(const float2 *__restrict__ tw, int k) {
+    return __ldg(tw + tw_offset(2, L) + k);
 }
 
-// A line's tables for passes 1..P-1 copied into shared memory.  Pass p's
-// table (L_p / R_p rows of R_p / 4 float4 vectors) is stored vector-major,
-// [vector h][row k], so the consecutive butterflies of a warp read
-// consecutive 16-byte words.  Needs R_p >= 4 for every p >= 1.
+// A line's tables for passes 1..P-1 copied into shared memory, in the global
+// tables' vector order (pass p: R_p / 4 vectors of L_p / R_p float4).  Needs
+// R_p >= 4 for every p >= 1.
 __host__ __device__ constexpr int tw_smem_offset4(int n, int p, int mb) {
     return p <= 1 ? 0
                   : tw_smem_offset4(n, p - 1, mb) + pass_span(n, p - 1, mb) * pass_radix(n, p - 1, mb) / 4;
@@ -235,16 +229,14 @@ struct SmemTw {
 };
 
 template <int N, int MB, int P_, int R, int L>
-__device__ __forceinline__ void tw_row(const SmemTw<N, MB> &tw, int k, float2 (&w)[R / 2]) {
+__device__ __forceinline__ float4 tw_pair(const SmemTw<N, MB> &tw, int k, int h) {
     static_assert(R >= 4, "shared-memory twiddles need radix >= 4");
-    constexpr int rows = L / R;
-    const float4 *w4 = tw.base + tw_smem_offset4(N, P_, MB) + k;
-#pragma unroll
-    for (int h = 0; h < R / 4; h++) {
-        const float4 q = w4[h * rows];
-        w[2 * h] = make_float2(q.x, q.y);
-        w[2 * h + 1] = make_float2(q.z, q.w);
-    }
+    return tw.base[tw_smem_offset4(N, P_, MB) + h * (L / R) + k];
+}
+template <int N, int MB, int P_, int L>
+__device__ __forceinline__ float2 tw_single(const SmemTw<N, MB> &, int) {
+    static_assert(N < 0, "a pass with radix 2 has no shared-memory table");
+    return make_float2(0.f, 0.f);
 }
 
 // Copy a line's tables from the global tables into `dst` (shared memory);
@@ -253,13 +245,10 @@ template <int N, int MB, int p>
 __device__ __forceinline__ void tw_fill_pass(float4 *dst, const float2 *__restrict__ tw, int tid,
                                              int nthreads) {
     if constexpr (p < num_passes(N, MB)) {
-        constexpr int R = pass_radix(N, p, MB), L = pass_span(N, p, MB) * R, rows = L / R;
+        constexpr int R = pass_radix(N, p, MB), L = pass_span(N, p, MB) * R;
         const float4 *src = reinterpret_cast<const float4 *>(tw + tw_offset(R, L));
         float4 *d = dst + tw_smem_offset4(N, p, MB);
-        for (int i = tid; i < rows * (R / 4); i += nthreads) {
-            const int k = i % rows, h = i / rows;
-            d[h * rows + k] = __ldg(src + k * (R / 2) + h);
-        }
+        for (int i = tid; i < L / 4; i += nthreads) d[i] = __ldg(src + i);
         tw_fill_pass<N, MB, p + 1>(dst, tw, tid, nthreads);
     }
 }
@@ -272,19 +261,17 @@ __device__ __forceinline__ void tw_fill_smem(float4 *dst, const float2 *__restri
 
 // Shared-memory accessors map a line position to a padded slot: the linear
 // index i (position * KW + column) gets one pad per 16, slot = i + i/16.
-// Strided<Sm, DELTA, COUNT> tells whether COUNT accesses DELTA positions
-// apart from a base are a fixed slot step apart (so one address and
-// compile-time offsets serve them all): true when the linear step is a
-// multiple of 16, or when all COUNT accesses fall inside one 16-slot block
-// (the base is then aligned to DELTA*COUNT*KW, as every caller's base is).
-template <class Sm, int DELTA, int COUNT>
-struct Strided {
-    static constexpr int LIN = DELTA * Sm::KW;
-    static constexpr bool by_block = (LIN % 16) == 0;
-    static constexpr bool in_block = LIN * COUNT <= 16;
-    static constexpr bool affine = by_block || in_block;
-    static constexpr int STEP = by_block ? LIN + LIN / 16 : LIN;
-};
+// slot_step: from a base access to the one r * DELTA positions on, for the
+// accesses of one butterfly or one thread's reads (base = a multiple of
+// DELTA * COUNT positions plus an offset below DELTA; all powers of two).
+// With LIN = DELTA * KW: a LIN of 16 or more adds whole pads; below that the
+// base's offset cannot carry into the next pad (it is below LIN), and the
+// base's multiple is whole pads or, when all accesses span less than 16,
+// never crosses one.  So one address and compile-time steps serve them all.
+template <class Sm, int DELTA>
+__host__ __device__ constexpr int slot_step(int r) {
+    return r * DELTA * Sm::KW + ((r * DELTA * Sm::KW) >> 4);
+}
 
 // Sm: shared-memory accessor for this thread's line: at(pos) -> float2*
 // (one exchange of complex values, KW as above), or, with Sm::kSplit,
@@ -328,18 +315,24 @@ struct LineFft {
                     // the twiddle loads (entry R/2 is stored in slot 0, whose
                     // value w^0 = 1 is never needed)
                     const int k = j & (Ns - 1);
-                    float2 w[R / 2];
-                    tw_row<N, MB, p, R, Ns * R>(tw, k, w);
                     if constexpr (R == 2) {
-                        v[1] = cmul(v[1], w[0]);
+                        v[1] = cmul(v[1], tw_single<N, MB, p, Ns * R>(tw, k));
                     } else {
-                        const float2 wh = w[0];  // w^(R/2)
+                        float2 wh = make_float2(1.f, 0.f);  // w^(R/2), from pair 0
 #pragma unroll
-                        for (int r = 1; r < R / 2; r++) {
-                            v[r] = cmul(v[r], w[r]);
-                            v[r + R / 2] = cmul(v[r + R / 2], cmul(wh, w[r]));
+                        for (int h = 0; h < R / 4; h++) {
+                            const float4 q = tw_pair<N, MB, p, R, Ns * R>(tw, k, h);
+                            const float2 w0 = make_float2(q.x, q.y), w1 = make_float2(q.z, q.w);
+                            if (h == 0) {
+                                wh = w0;
+                                v[R / 2] = cmul(v[R / 2], wh);
+                            } else {
+                                v[2 * h] = cmul(v[2 * h], w0);
+                                v[2 * h + R / 2] = cmul(v[2 * h + R / 2], cmul(wh, w0));
+                            }
+                            v[2 * h + 1] = cmul(v[2 * h + 1], w1);
+                            v[2 * h + 1 + R / 2] = cmul(v[2 * h + 1 + R / 2], cmul(wh, w1));
                         }
-                        v[R / 2] = cmul(v[R / 2], wh);
                     }
                 }
                 Dft<R>::run(v);
@@ -348,15 +341,9 @@ struct LineFft {
                     for (int r = 0; r < R; r++) x[s + r * S] = v[r];
                 } else {
                     const int d = (j / Ns) * Ns * R + (j & (Ns - 1));
-                    using WS = Strided<Sm, Ns, R>;
-                    if constexpr (WS::affine) {
-                        float2 *o = sm.at(d);
+                    float2 *o = sm.at(d);
 #pragma unroll
-                        for (int r = 0; r < R; r++) o[r * WS::STEP] = v[r];
-                    } else {
-#pragma unroll
-                        for (int r = 0; r < R; r++) *sm.at(d + r * Ns) = v[r];
-                    }
+                    for (int r = 0; r < R; r++) o[slot_step<Sm, Ns>(r)] = v[r];
                 }
             }
             if constexpr (!last && Sm::kSplit) {
@@ -365,15 +352,9 @@ struct LineFft {
                 pass<p + 1>(x, t, sm, tw);
             } else if constexpr (!last) {
                 sync();
-                using RS = Strided<Sm, T, E>;
-                if constexpr (RS::affine) {
-                    const float2 *in = sm.at(t);
+                const float2 *in = sm.at(t);
 #pragma unroll
-                    for (int m = 0; m < E; m++) x[m] = in[m * RS::STEP];
-                } else {
-#pragma unroll
-                    for (int m = 0; m < E; m++) x[m] = *sm.at(t + m * T);
-                }
+                for (int m = 0; m < E; m++) x[m] = in[slot_step<Sm, T>(m)];
                 // the next exchange overwrites the buffer; after the last one
                 // the caller syncs before it writes the buffer again
                 if constexpr (p + 2 < P) sync();
