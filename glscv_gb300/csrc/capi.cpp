@@ -564,12 +564,14 @@ int glsfft_phase_correlate_async(glsfft_context ctx, const float *src1, const fl
                       d_result, (cudaStream_t)stream);
 }
 
-// The synchronous call's three launches into the context's mapped result:
-// a replay of the cached graph when the call repeats the last one's
-// buffers, shape and workspace (one graph launch instead of three kernel
-// launches), else the launches captured into a new graph on the context's
-// private stream and that graph launched; if the capture is refused, the
-// launches themselves.
+// The synchronous call's three launches into the context's mapped result.
+// A call that repeats the last one's buffers, shape and workspace replays
+// them as one CUDA graph, captured at the first repeat on the context's
+// private stream (if the capture is refused, the launches themselves).  A
+// call with other buffers -- the frames of a video loop alternate -- makes
+// the three launches directly: capturing and instantiating a graph for each
+// such call cost more host time than the pipeline takes (GB300, 1024^2 with
+// changing buffers: 60 us per call with the capture, 33 us without).
 static int poc_sync_launch(glsfft_context ctx, const float *src1, const float *src2,
                            const float *window, int rows, int cols, int box, cudaStream_t s) {
     const size_t n = (size_t)rows * cols;
@@ -587,12 +589,16 @@ static int poc_sync_launch(glsfft_context ctx, const float *src1, const float *s
     ctx->surface_count = n;
     auto &pg = ctx->poc_graph;
     auto same = [&] {
-        return pg.exec && pg.src1 == src1 && pg.src2 == src2 && pg.window == window &&
+        return pg.src1 == src1 && pg.src2 == src2 && pg.window == window &&
                pg.rows == rows && pg.cols == cols && pg.box == box && pg.ws == ctx->ws;
     };
     if (!same()) {
         if (pg.exec) cudaGraphExecDestroy(pg.exec);
-        pg = glsfft_context_s::PocGraph{};
+        pg = {src1, src2, window, rows, cols, box, ctx->ws, nullptr};
+        return poc_launch(ctx->d_tw, src1, src2, window, rows, cols, box, f1, f2, surface, key,
+                          ctx->h_result_dev, s, flag);
+    }
+    if (!pg.exec) {  // the first repeat
         if (!ctx->capture_stream &&
             cudaStreamCreateWithFlags(&ctx->capture_stream, cudaStreamNonBlocking) != cudaSuccess)
             ctx->capture_stream = nullptr;
@@ -603,14 +609,14 @@ static int poc_sync_launch(glsfft_context ctx, const float *src1, const float *s
             st = poc_launch(ctx->d_tw, src1, src2, window, rows, cols, box, f1, f2, surface, key,
                             ctx->h_result_dev, ctx->capture_stream, flag);
             const cudaError_t e = cudaStreamEndCapture(ctx->capture_stream, &graph);
-            cudaGraphExec_t exec = nullptr;
-            if (!st && e == cudaSuccess && graph && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess)
-                pg = {src1, src2, window, rows, cols, box, ctx->ws, exec};
+            if (st || e != cudaSuccess || !graph ||
+                cudaGraphInstantiate(&pg.exec, graph, 0) != cudaSuccess)
+                pg.exec = nullptr;
             if (graph) cudaGraphDestroy(graph);
         }
         cudaGetLastError();  // a refused capture leaves no error behind
     }
-    if (same()) return cuda_status(cudaGraphLaunch(pg.exec, s));
+    if (pg.exec) return cuda_status(cudaGraphLaunch(pg.exec, s));
     return poc_launch(ctx->d_tw, src1, src2, window, rows, cols, box, f1, f2, surface, key,
                       ctx->h_result_dev, s, flag);
 }

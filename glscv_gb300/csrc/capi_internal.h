@@ -33,8 +33,8 @@ struct glsfft_context_s {
     long long stall_ns = 0;   // glsfft_context_inject_stall (0: off)
     // the reference-arithmetic mode's twiddle tables, per line length
     std::map<int, float2 *> exact_tw;
-    // glsfft_phase_correlate's three launches as a CUDA graph, replayed
-    // while a call repeats the last one's buffers, shape and workspace
+    // the last glsfft_phase_correlate call's buffers, shape and workspace,
+    // and, once a call has repeated them, its three launches as a CUDA graph
     struct PocGraph {
         const float *src1 = nullptr, *src2 = nullptr, *window = nullptr;
         int rows = 0, cols = 0, box = 0;
