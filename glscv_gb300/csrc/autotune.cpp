@@ -171,6 +171,7 @@ int glsfft_autotune_fft2d(glsfft_context ctx, int rows, int cols, int count,
     a.scale = 1.0f;
     a.tw = ctx->d_tw;
     a.in_img_bytes = a.out_img_bytes = (size_t)rows * cols * sizeof(float2);
+    a.spread = 1;
     // each pass: its default schedule first, then the others in order; the
     // fastest is kept unless the default is within kKeepMargin of it
     const FftSchedule dflt = default_schedule(rows, cols);

@@ -159,6 +159,16 @@ DeviceGuard::~DeviceGuard() {
     if (prev_ >= 0 && cudaGetDevice(&cur) == cudaSuccess && cur != prev_) cudaSetDevice(prev_);
 }
 
+int glsfft::sm_count() {
+    static std::atomic<int> known[64];  // zero-initialised
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 0;
+    if (dev < 64 && (n = known[dev].load(std::memory_order_relaxed))) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    if (dev < 64) known[dev].store(n, std::memory_order_relaxed);
+    return n;
+}
+
 cudaError_t glsfft::smem_opt_in(const void *kern, size_t bytes) {
     static std::mutex mu;
     static std::set<std::pair<const void *, int>> done;
@@ -223,7 +233,7 @@ int glsfft::fft2d_launch(glsfft_context ctx, const void *src, void *dst, int row
         a.stall_ns = ctx->stall_ns;
         a.in_img_bytes = px * (real_in ? sizeof(float) : sizeof(float2));
         a.out_img_bytes = px * sizeof(float2);
-        a.pdl = 1;
+        a.pdl = a.spread = 1;
         cudaError_t e = real_in ? launch_rows(cols, LD_R1, ST_C2, a, count, s)
                                 : launch_rows_sched(cols, sc.row, a, count, s);
         if (e != cudaSuccess) return cuda_status(e);
@@ -241,7 +251,7 @@ int glsfft::fft2d_launch(glsfft_context ctx, const void *src, void *dst, int row
         a.err = ctx->d_status;
         a.stall_ns = ctx->stall_ns;
         a.in_img_bytes = a.out_img_bytes = px * sizeof(float2);
-        a.pdl = 1;
+        a.pdl = a.spread = 1;
         cudaError_t e = launch_cols_sched(rows, sc.col, a, count, s);
         if (e != cudaSuccess) return cuda_status(e);
     }
@@ -269,7 +279,7 @@ int glsfft::poc_launch(const float2 *tw, const float *src1, const float *src2,
     a.cols = cols;
     a.scale = 1.0f;
     a.tw = tw;
-    a.pdl = 1;
+    a.pdl = a.spread = 1;
     cudaError_t e = launch_rows(cols, window ? LD_R1W : LD_R1, ST_C2, a, 2, s);
     if (e != cudaSuccess) return cuda_status(e);
 
@@ -282,7 +292,7 @@ int glsfft::poc_launch(const float2 *tw, const float *src1, const float *src2,
     b.scale = 1.0f;
     b.key = key;
     b.tw = tw;
-    b.pdl = 1;
+    b.pdl = b.spread = 1;
     e = launch_poc_cols(rows, b, s);
     if (e != cudaSuccess) return cuda_status(e);
 
@@ -298,7 +308,7 @@ int glsfft::poc_launch(const float2 *tw, const float *src1, const float *src2,
     c.result = d_result;
     c.box = box;
     c.done_flag = done_flag;
-    c.pdl = 1;
+    c.pdl = c.spread = 1;
     e = launch_rows(cols, LD_C2, ST_RE_ARGMAX, c, 1, s);
     return cuda_status(e);
 }
@@ -511,7 +521,8 @@ static int one_pass(glsfft_context ctx, const void *src, void *dst, int count, i
               ((flags & GLSFFT_SHIFT) ? (along_rows ? PF_SHIFT_COLS : PF_SHIFT_ROWS) : 0u);
     a.tw = ctx->d_tw;
     a.err = ctx->d_status;
-        a.stall_ns = ctx->stall_ns;
+    a.stall_ns = ctx->stall_ns;
+    a.spread = 1;
     a.in_img_bytes = a.out_img_bytes = (size_t)rows * cols * sizeof(float2);
     const FftSchedule sc = schedule_for(ctx->sched, rows, cols);
     cudaError_t e = along_rows ? launch_rows_sched(n, sc.row, a, count, s)

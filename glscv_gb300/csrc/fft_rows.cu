@@ -13,19 +13,33 @@ constexpr PassShape rows_fixed_shape() {
     return (N >= 2048 && !(LD == LD_C2 && ST == ST_C2)) ? row_shape(N, 2) : row_shape(N, 0);
 }
 
+// Rows per block.  Grids of many blocks take the fixed shape's; a grid that
+// would leave SMs idle or unevenly loaded takes the SMs' even share of its
+// rows instead, in one block per SM where that fits 512 threads: 1024 rows
+// are 147 blocks of 7 (one per SM), where 256 blocks of 4 load some SMs with
+// 8 rows, and 512 rows of 512 points 128 blocks of 4 rather than 64 of 8.
+// Whole warps only.
+static int row_lines(int fixed, int threads_per_line, int max_lines, long long total) {
+    const int sms = sm_count();
+    if (sms <= 0 || total >= 4LL * fixed * sms) return fixed;
+    const int unit = threads_per_line < 32 ? 32 / threads_per_line : 1;
+    for (int k = 1;; k++) {
+        int lines = (int)((total + (long long)sms * k - 1) / ((long long)sms * k));
+        lines = (lines + unit - 1) / unit * unit;
+        if (lines <= max_lines) return lines;
+    }
+}
+
 template <int N, int LD, int ST>
 static cudaError_t rows_t(const PassArgs &a, int images, cudaStream_t s) {
     constexpr PassShape sh = rows_fixed_shape<N, LD, ST>();
-    constexpr int E = sh.E, LINES = sh.G, T = N / E;
-    constexpr int threads = LINES * T;
-    constexpr size_t smem = num_passes(N) > 1 ? sizeof(float2) * (size_t)LINES * padded_count(N) : 0;
-    auto kern = fft_rows_kernel<N, E, LINES, LD, ST, sh.MB>;
-    if constexpr (smem > 48 * 1024) {
-        const cudaError_t e = smem_opt_in(reinterpret_cast<const void *>(kern), smem);
-        if (e != cudaSuccess) return e;
-    }
-    dim3 grid((a.rows + LINES - 1) / LINES, images);
-    return launch_pass(kern, grid, threads, smem, s, a);
+    constexpr int E = sh.E, T = N / E, MAXL = cmax(sh.G, 512 / T);
+    const int lines = a.spread ? row_lines(sh.G, T, MAXL, (long long)a.rows * images) : sh.G;
+    const size_t smem =
+        num_passes(N) > 1 ? sizeof(float2) * (size_t)lines * padded_count(N) : 0;
+    auto kern = fft_rows_kernel<N, E, MAXL, LD, ST, sh.MB>;
+    dim3 grid((a.rows + lines - 1) / lines, images);
+    return launch_pass(kern, grid, lines * T, smem, s, a);
 }
 
 template <int LD, int ST>

@@ -75,6 +75,8 @@ struct PassArgs {
     // leaves its first tile's copy unissued and waits this many nanoseconds
     // for it, so the wait runs out
     long long stall_ns;
+    // a small grid is spread evenly over the SMs (launch_pass)
+    int spread;
     // launch with programmatic dependent launch (every pass kernel begins
     // with griddepcontrol.wait): the grid may become resident before its
     // stream predecessor ends
@@ -101,6 +103,9 @@ cudaError_t launch_stream_pass(int n, bool cols, const PassArgs &a, int images, 
 // copies (batch.cpp).  GLSFFT_SUCCESS or an error status.
 int make_tmap_2d(void *tmap128, const void *base, long long width, long long height, int box_w,
                  int box_h);
+
+// SMs of the current device (0 on failure), looked up once per device.
+int sm_count();
 
 // Opt kernel `kern` into `bytes` of dynamic shared memory on the current
 // device.  The attribute belongs to the kernel's instance on one device, so

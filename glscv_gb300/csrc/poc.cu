@@ -11,10 +11,6 @@ static cudaError_t poc_t(const PassArgs &a, cudaStream_t s) {
     constexpr int threads = W * T;
     constexpr size_t smem = num_passes(N) > 1 ? sizeof(float2) * (size_t)padded_count(N * W) : 0;
     auto kern = poc_cols_kernel<N, E, W>;
-    if constexpr (smem > 48 * 1024) {
-        const cudaError_t e = smem_opt_in(reinterpret_cast<const void *>(kern), smem);
-        if (e != cudaSuccess) return e;
-    }
     dim3 grid((a.cols + W - 1) / W, 1);
     return launch_pass(kern, grid, threads, smem, s, a);
 }

@@ -440,7 +440,7 @@ int glsfft_fft_display(glsfft_context ctx, const float *frame, const float *wind
     r.flags = PF_SHIFT_COLS;
     r.tw = ctx->d_tw;
     r.key = keys;
-    r.pdl = 1;  // the three launches are chained by programmatic dependent launch
+    r.pdl = r.spread = 1;  // the three launches are chained by programmatic dependent launch
     cudaError_t e = launch_rows(cols, window ? LD_R1W : LD_R1, ST_C2, r, 1, s);
     if (e != cudaSuccess) return cuda_status(e);
     if (rows > 1) {
@@ -457,7 +457,7 @@ int glsfft_fft_display(glsfft_context ctx, const float *frame, const float *wind
         c.param = offset;
         c.err = ctx->d_status;
         c.stall_ns = ctx->stall_ns;
-        c.pdl = 1;  // the plain column kernel; the streamed pass launches as usual
+        c.pdl = c.spread = 1;  // the plain column kernel; the streamed pass launches as usual
         // 4096-point columns: the streamed pass (TMA-fed, one block per SM)
         e = rows == 4096 && stream_pass_applies(rows, true, c, 1, ST_LOGMAG_MINMAX)
                 ? launch_stream_pass(rows, true, c, 1, s, ST_LOGMAG_MINMAX)
