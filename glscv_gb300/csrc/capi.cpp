@@ -219,6 +219,20 @@ int glsfft::fft2d_launch(glsfft_context ctx, const void *src, void *dst, int row
     const bool do_cols = rows > 1;
     const size_t px = (size_t)rows * cols;
     const FftSchedule sc = schedule_for(ctx->sched, rows, cols);
+    if (sc.row == 0 && sc.col == 0 && fused_applies(rows, cols)) {
+        PassArgs a{};
+        a.in0 = src;
+        a.out0 = dst;
+        a.rows = rows;
+        a.cols = cols;
+        a.scale = scale ? 1.0f / (float)cols : 1.0f;
+        a.flags = (inv ? PF_CONJ_IN | PF_CONJ_OUT : 0u) |
+                  (shift ? PF_SHIFT_ROWS | PF_SHIFT_COLS : 0u);
+        a.tw = ctx->d_tw;
+        a.in_img_bytes = px * (real_in ? sizeof(float) : sizeof(float2));
+        a.out_img_bytes = px * sizeof(float2);
+        return cuda_status(launch_fused(a, real_in, scale ? 1.0f / (float)rows : 1.0f, count, s));
+    }
     if (do_rows) {
         PassArgs a{};
         a.in0 = src;

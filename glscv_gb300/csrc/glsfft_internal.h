@@ -89,6 +89,14 @@ cudaError_t launch_rows(int n, int ld, int st, const PassArgs &a, int images, cu
 cudaError_t launch_cols(int n, int ld, int st, const PassArgs &a, int images, cudaStream_t s);
 cudaError_t launch_poc_cols(int n, const PassArgs &a, cudaStream_t s);
 
+// A whole 2-D FFT in one launch (fft_fused.cu): whether the image size is
+// one it takes, and the launch over `images` contiguous images -- in0, out0,
+// rows, cols, tw, in_img_bytes, both passes' flags, `scale` after the rows
+// and `scale_cols` after the columns; real_in: in0 holds CV_32FC1 images.
+bool fused_applies(int rows, int cols);
+cudaError_t launch_fused(const PassArgs &a, bool real_in, float scale_cols, int images,
+                         cudaStream_t s);
+
 // The streamed column pass for 2048- and 4096-point columns (fft_stream.cu;
 // cols must be true): whether it applies to these arguments (contiguous
 // complex images, 16-byte aligned, the column count a multiple of the

@@ -97,7 +97,8 @@ GLSFFT_API int glsfft_context_inject_stall(glsfft_context ctx, long long wait_li
 /*
  * 2-D complex FFT of a CV_32FC2 rows x cols device image:
  * gls::fft(src, dst, flag), glsCV/glsFft.h:55 / glsFft.cpp:675-708.
- * Rows pass then columns pass, one kernel each.  src == dst is allowed
+ * Rows pass then columns pass, one kernel each (one kernel for both up to 4096
+ * pixels).  src == dst is allowed
  * (in-place, as glsPhaseCorrelate.cpp:199 uses it).  Asynchronous on
  * `stream`; uses no workspace.
  */
@@ -202,7 +203,9 @@ GLSFFT_API int glsfft_schedule_available(int length, int schedule, int along_col
  * rows x cols images on this context.  Until set or tuned, a size runs its
  * built-in default, measured on GB300: row schedule 2 for 2048- and
  * 4096-point rows, the streamed column pass for 4096-point columns,
- * schedule 0 otherwise. */
+ * schedule 0 otherwise; images of 16 points a side and more and at most 4096
+ * pixels run both passes of fft2d / fft2d_batched in one launch (bit-identical
+ * to schedules 0, 0) until another pair is set. */
 GLSFFT_API int glsfft_set_fft_schedule(glsfft_context ctx, int rows, int cols, int row_schedule,
                                        int col_schedule);
 GLSFFT_API int glsfft_get_fft_schedule(glsfft_context ctx, int rows, int cols,
