@@ -275,7 +275,8 @@ __host__ __device__ constexpr int slot_step(int r) {
 
 // Sm: shared-memory accessor for this thread's line: at(pos) -> float2*
 // (one exchange of complex values, KW as above), or, with Sm::kSplit,
-// at<X>(pos) -> float* for the exchange after pass X (the exchange runs
+// at<X>(pos) -> float* and step(dpos), the slots from a base access to the one
+// dpos positions on (as slot_step), for the exchange after pass X (the exchange runs
 // twice through a buffer half the size, real parts then imaginary parts;
 // each exchange may pad differently, as its stores and loads are its own).
 // tw: the per-pass twiddle tables above.
@@ -378,14 +379,15 @@ struct LineFft {
         for (int s = 0; s < S; s++) {
             const int j = t + s * T;
             const int d = (j / Ns) * Ns * R + (j & (Ns - 1));
+            float *o = sm.template at<p>(d);
 #pragma unroll
-            for (int r = 0; r < R; r++)
-                *sm.template at<p>(d + r * Ns) = H ? x[s + r * S].y : x[s + r * S].x;
+            for (int r = 0; r < R; r++) o[Sm::step(r * Ns)] = H ? x[s + r * S].y : x[s + r * S].x;
         }
         sync();
+        const float *in = sm.template at<p>(t);
 #pragma unroll
         for (int m = 0; m < E; m++) {
-            const float v = *sm.template at<p>(t + m * T);
+            const float v = in[Sm::step(m * T)];
             if constexpr (H == 0) x[m].x = v;
             else x[m].y = v;
         }
