@@ -3,6 +3,7 @@
 // gls::phaseCorrelate.
 #include "glsfft.h"
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cmath>
@@ -398,6 +399,10 @@ int glsfft_context_create(glsfft_context *out, int device) {
     if (e == cudaSuccess) e = cudaHostGetDevicePointer(&ctx->h_result_dev, ctx->h_result, 0);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_status, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(ctx->d_status, 0, sizeof(int));
+    if (e == cudaSuccess) {
+        ctx->key_pairs = 8 * std::max(sm_count(), 1);
+        e = cudaMalloc(&ctx->d_keys, 16 * (size_t)ctx->key_pairs);
+    }
     int st = cuda_status(e);
     if (!st) st = tc_tables_create(&ctx->tc);
     if (st) {
@@ -405,6 +410,7 @@ int glsfft_context_create(glsfft_context *out, int device) {
         if (ctx->d_tw) cudaFree(ctx->d_tw);
         if (ctx->h_result) cudaFreeHost(ctx->h_result);
         if (ctx->d_status) cudaFree(ctx->d_status);
+        if (ctx->d_keys) cudaFree(ctx->d_keys);
         delete ctx;
         return st;
     }
@@ -422,6 +428,7 @@ int glsfft_context_destroy(glsfft_context ctx) {
     if (ctx->d_tw) cudaFree(ctx->d_tw);
     if (ctx->h_result) cudaFreeHost(ctx->h_result);
     if (ctx->d_status) cudaFree(ctx->d_status);
+    if (ctx->d_keys) cudaFree(ctx->d_keys);
     for (auto &t : ctx->exact_tw) cudaFree(t.second);
     tc_tables_destroy(&ctx->tc);
     delete ctx;

@@ -29,6 +29,10 @@ struct glsfft_context_s {
     // launches use; sizes not listed run schedule 0
     std::map<long long, glsfft::FftSchedule> sched;
     HostPipe *host_pipe = nullptr;  // glsfft_fft2d_host's pipeline, built on first use
+    // key pairs of the normalisation's min / max blocks: one for every block
+    // of 256 threads that fits the device
+    unsigned long long *d_keys = nullptr;
+    int key_pairs = 0;
     int *d_status = nullptr;  // device status word of bounded waits (glsfft_device_status)
     long long stall_ns = 0;   // glsfft_context_inject_stall (0: off)
     // the reference-arithmetic mode's twiddle tables, per line length

@@ -14,6 +14,8 @@
 //   glsCam FFT view        glsCam/glsCam.cpp:196-203
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cstdint>
 
 #include "capi_internal.h"
@@ -31,21 +33,25 @@ constexpr int kThreads = 256;
 
 // Blocks for n elements: one wave of the kernel's resident blocks at most
 // (grid-stride beyond).  A grid of more blocks than fit at once would run a
-// partial second wave at a fraction of the occupancy.
-template <class Kernel>
-int grid_for(Kernel kern, size_t n) {
-    int dev = 0, sms = 0, per_sm = 0;
+// partial second wave at a fraction of the occupancy.  KERN's resident blocks
+// are looked up once per device.
+template <auto KERN>
+int grid_for(size_t n) {
+    static std::atomic<int> known[64];  // resident blocks per device, 0 = not looked up
+    int dev = 0, cap = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, 0) != cudaSuccess) {
-        cudaGetLastError();
-        per_sm = 1;
+    if (dev >= 0 && dev < 64) cap = known[dev].load(std::memory_order_relaxed);
+    if (!cap) {
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KERN, kThreads, 0) != cudaSuccess) {
+            cudaGetLastError();
+            per_sm = 1;
+        }
+        cap = std::max(sm_count(), 1) * std::max(per_sm, 1);
+        if (dev >= 0 && dev < 64) known[dev].store(cap, std::memory_order_relaxed);
     }
-    if (sms <= 0) sms = 1;
-    if (per_sm <= 0) per_sm = 1;
     const size_t want = (n + kThreads - 1) / kThreads;
-    const size_t cap = (size_t)sms * per_sm;
-    return (int)(want < cap ? (want ? want : 1) : cap);
+    return (int)(want < (size_t)cap ? (want ? want : 1) : (size_t)cap);
 }
 
 // The element kernels move 16 bytes per load and store (two complex or four
@@ -65,6 +71,7 @@ __device__ __forceinline__ float2 spec_binary_op(float2 x, float2 y) {
 template <int OP>
 __global__ void __launch_bounds__(kThreads) spec_binary_kernel(const float2 *a, const float2 *b,
                                                               float2 *d, size_t n) {
+    pdl_enter();
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     size_t done = 0;
@@ -109,6 +116,7 @@ __global__ void __launch_bounds__(kThreads) spec_mag_kernel(const float2 *__rest
                                                            unsigned long long *keys) {
     __shared__ unsigned long long red[2 * (kThreads / 32)];
     unsigned long long kmin = 0, kmax = 0;
+    pdl_enter();
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     size_t done = 0;
@@ -178,14 +186,20 @@ __global__ void minmax_reset_kernel(unsigned long long *keys) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// The input was complete before the reset kernel started (stream order);
-// only the keys come from it, so the pass waits for its predecessor grid
-// (griddepcontrol.wait, a no-op without programmatic launch) just before it
-// commits them.
+// PARTIAL = false: after minmax_reset_kernel, the keys are reduced over the
+// grid by atomics.  The input was complete before the reset kernel started
+// (stream order); only the keys come from it, so the pass waits for its
+// predecessor grid (griddepcontrol.wait, a no-op without programmatic launch)
+// just before it commits them.
+// PARTIAL = true: block b leaves its two keys in keys[2b], keys[2b + 1], for
+// a reader that reduces them itself (normalize_kernel): no reset and no
+// atomics.  The input may come from the grid before, so the wait comes first.
+template <bool PARTIAL>
 __global__ void __launch_bounds__(kThreads) minmax_kernel(const float *__restrict__ x, size_t n,
                                                           unsigned long long *keys) {
     __shared__ unsigned long long red[2 * (kThreads / 32)];
     MinMaxRun run;
+    if constexpr (PARTIAL) pdl_enter();
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     size_t done = 0;
@@ -216,42 +230,72 @@ __global__ void __launch_bounds__(kThreads) minmax_kernel(const float *__restric
         done = nv * 4;
     }
     for (size_t i = done + tid; i < n; i += stride) run.add(x[i], (unsigned)i);
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // the keys are reset
-    run.commit(red, keys);
+    if constexpr (PARTIAL) {
+        const ulonglong2 k = block_minmax(min_key(run.vmin, run.imin), max_key(run.vmax, run.imax), red);
+        if (threadIdx.x == 0) reinterpret_cast<ulonglong2 *>(keys)[blockIdx.x] = k;
+    } else {
+        asm volatile("griddepcontrol.wait;" ::: "memory");  // the keys are reset
+        run.commit(red, keys);
+    }
 }
 
 // dst = (float)(alpha - scl*min) + scl*src, scl = (float)(beta-alpha) / (float)(max-min)
+// The keys are `parts` pairs, the result their extremes.  Before the grid in
+// front (which made them) is over, a block already has its first values: the
+// source is complete when that grid runs (it reads it), and an in-place
+// destination is written only after the wait.
+// RAW: the source is written by the grid in front (the FFT display's column
+// pass), so the values wait too.
+template <bool RAW>
 __global__ void __launch_bounds__(kThreads) normalize_kernel(const float *x, float *d, size_t n,
                                                              const unsigned long long *keys,
-                                                             double alpha, double beta) {
-    pdl_enter();  // the keys come from the grid before
-    const double mn = min_key_value(keys[0]), mx = max_key_value(keys[1]);
-    const float scl = __fdiv_rn((float)(beta - alpha), (float)(mx - mn));
-    const float c = (float)__dsub_rn(alpha, __dmul_rn((double)scl, mn));
+                                                             int parts, double alpha, double beta) {
+    __shared__ unsigned long long red[2 * (kThreads / 32)];
+    __shared__ ulonglong2 s_key;
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
-    size_t done = 0;
-    if (al16(x) && al16(d)) {
-        const size_t nv = n / 4;
-        const float4 *x4 = reinterpret_cast<const float4 *>(x);
-        float4 *d4 = reinterpret_cast<float4 *>(d);
-        auto step = [&](const float4 v) {
-            return make_float4(__fadd_rn(c, __fmul_rn(scl, v.x)), __fadd_rn(c, __fmul_rn(scl, v.y)),
-                               __fadd_rn(c, __fmul_rn(scl, v.z)), __fadd_rn(c, __fmul_rn(scl, v.w)));
-        };
-        // four loads in flight; the last batch predicated (one round trip)
-        for (size_t i = tid; i < nv; i += 4 * stride) {
-            float4 v[4];
+    const bool vec = al16(x) && al16(d);
+    const size_t nv = vec ? n / 4 : 0;
+    const float4 *x4 = reinterpret_cast<const float4 *>(x);
+    float4 *d4 = reinterpret_cast<float4 *>(d);
+    constexpr int kBatch = 4;  // loads in flight; the last batch predicated (one round trip)
+    float4 v[kBatch];
+    auto fetch = [&](size_t i) {
 #pragma unroll
-            for (int k = 0; k < 4; k++)
-                v[k] = i + k * stride < nv ? x4[i + k * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-                if (i + k * stride < nv) d4[i + k * stride] = step(v[k]);
-        }
-        done = nv * 4;
+        for (int k = 0; k < kBatch; k++)
+            v[k] = i + k * stride < nv ? x4[i + k * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    if constexpr (RAW) pdl_enter();
+    fetch(tid);
+    if constexpr (!RAW) pdl_enter();
+    unsigned long long kmin = 0, kmax = 0;
+    for (int i = threadIdx.x; i < parts; i += kThreads) {
+        const ulonglong2 k = __ldcg(reinterpret_cast<const ulonglong2 *>(keys) + i);
+        kmin = k.x > kmin ? k.x : kmin;
+        kmax = k.y > kmax ? k.y : kmax;
     }
-    for (size_t i = done + tid; i < n; i += stride) d[i] = __fadd_rn(c, __fmul_rn(scl, x[i]));
+    if (parts > 1) {
+        const ulonglong2 k = block_minmax(kmin, kmax, red);
+        if (threadIdx.x == 0) s_key = k;
+    } else if (threadIdx.x == 0) {
+        s_key = make_ulonglong2(kmin, kmax);
+    }
+    __syncthreads();
+    const double mn = min_key_value(s_key.x), mx = max_key_value(s_key.y);
+    const float scl = __fdiv_rn((float)(beta - alpha), (float)(mx - mn));
+    const float c = (float)__dsub_rn(alpha, __dmul_rn((double)scl, mn));
+    auto step = [&](const float4 q) {
+        return make_float4(__fadd_rn(c, __fmul_rn(scl, q.x)), __fadd_rn(c, __fmul_rn(scl, q.y)),
+                           __fadd_rn(c, __fmul_rn(scl, q.z)), __fadd_rn(c, __fmul_rn(scl, q.w)));
+    };
+    for (size_t i = tid; i < nv;) {
+#pragma unroll
+        for (int k = 0; k < kBatch; k++)
+            if (i + k * stride < nv) d4[i + k * stride] = step(v[k]);
+        i += kBatch * stride;
+        if (i < nv) fetch(i);
+    }
+    for (size_t i = nv * 4 + tid; i < n; i += stride) d[i] = __fadd_rn(c, __fmul_rn(scl, x[i]));
 }
 
 bool misaligned(const void *p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) != 0; }
@@ -294,11 +338,12 @@ int glsfft_mul_spectrums(glsfft_context ctx, const void *src0, const void *src1,
     const auto *b = static_cast<const float2 *>(src1);
     auto *d = static_cast<float2 *>(dst);
     cudaStream_t s = (cudaStream_t)stream;
-    if (conj)
-        spec_binary_kernel<1><<<grid_for(spec_binary_kernel<1>, n), kThreads, 0, s>>>(a, b, d, n);
-    else
-        spec_binary_kernel<0><<<grid_for(spec_binary_kernel<0>, n), kThreads, 0, s>>>(a, b, d, n);
-    return cuda_status(cudaGetLastError());
+    // every element kernel is launched as its predecessor's programmatic
+    // dependent: resident while that drains
+    return cuda_status(conj ? launch_maybe_pdl(true, spec_binary_kernel<1>, grid_for<spec_binary_kernel<1>>(n),
+                                               kThreads, 0, s, a, b, d, n)
+                            : launch_maybe_pdl(true, spec_binary_kernel<0>, grid_for<spec_binary_kernel<0>>(n),
+                                               kThreads, 0, s, a, b, d, n));
 }
 
 int glsfft_mul_spectrums_phase_only(glsfft_context ctx, const void *src0, const void *src1,
@@ -309,11 +354,10 @@ int glsfft_mul_spectrums_phase_only(glsfft_context ctx, const void *src0, const 
     DeviceGuard g(ctx->device);
     if (!g.ok()) return GLSFFT_ERROR_CUDA;
     const size_t n = (size_t)rows * cols;
-    auto kern = spec_binary_kernel<2>;
-    kern<<<grid_for(kern, n), kThreads, 0, (cudaStream_t)stream>>>(
-        static_cast<const float2 *>(src0), static_cast<const float2 *>(src1),
-        static_cast<float2 *>(dst), n);
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launch_maybe_pdl(true, spec_binary_kernel<2>, grid_for<spec_binary_kernel<2>>(n),
+                                        kThreads, 0, (cudaStream_t)stream,
+                                        static_cast<const float2 *>(src0),
+                                        static_cast<const float2 *>(src1), static_cast<float2 *>(dst), n));
 }
 
 int glsfft_mag_spectrums(glsfft_context ctx, const void *src, float *dst, int rows, int cols,
@@ -328,9 +372,9 @@ int glsfft_mag_spectrums(glsfft_context ctx, const void *src, float *dst, int ro
     if (!g.ok()) return GLSFFT_ERROR_CUDA;
     const size_t n = (size_t)rows * cols;
     auto kern = spec_mag_kernel<false, false>;
-    kern<<<grid_for(kern, n), kThreads, 0, (cudaStream_t)stream>>>(
-        static_cast<const float2 *>(src), dst, n, 0.0f, nullptr);
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launch_maybe_pdl(true, kern, grid_for<spec_mag_kernel<false, false>>(n), kThreads, 0,
+                                        (cudaStream_t)stream, static_cast<const float2 *>(src), dst, n,
+                                        0.0f, nullptr));
 }
 
 int glsfft_log_mag_spectrums(glsfft_context ctx, const void *src, float *dst, int rows, int cols,
@@ -344,9 +388,9 @@ int glsfft_log_mag_spectrums(glsfft_context ctx, const void *src, float *dst, in
     if (!g.ok()) return GLSFFT_ERROR_CUDA;
     const size_t n = (size_t)rows * cols;
     auto kern = spec_mag_kernel<true, false>;
-    kern<<<grid_for(kern, n), kThreads, 0, (cudaStream_t)stream>>>(
-        static_cast<const float2 *>(src), dst, n, offset, nullptr);
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launch_maybe_pdl(true, kern, grid_for<spec_mag_kernel<true, false>>(n), kThreads, 0,
+                                        (cudaStream_t)stream, static_cast<const float2 *>(src), dst, n,
+                                        offset, nullptr));
 }
 
 int glsfft_min_max_loc_async(glsfft_context ctx, const float *src, int rows, int cols,
@@ -360,7 +404,7 @@ int glsfft_min_max_loc_async(glsfft_context ctx, const float *src, int rows, int
     minmax_reset_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(d_keys);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_status(e);
-    return cuda_status(launch_maybe_pdl(true, minmax_kernel, grid_for(minmax_kernel, n / 4),
+    return cuda_status(launch_maybe_pdl(true, minmax_kernel<false>, grid_for<minmax_kernel<false>>(n / 4),
                                         kThreads, 0, (cudaStream_t)stream, src, n, d_keys));
 }
 
@@ -401,15 +445,20 @@ int glsfft_normalize_minmax(glsfft_context ctx, const float *src, float *dst, in
     if (st) return st;
     DeviceGuard g(ctx->device);
     if (!g.ok()) return GLSFFT_ERROR_CUDA;
-    unsigned long long *keys = nullptr;
-    st = keys_at(ctx, 0, &keys);
-    if (!st) st = glsfft_min_max_loc_async(ctx, src, rows, cols, keys, stream);
-    if (st) return st;
     const size_t n = (size_t)rows * cols;
-    // resident while the min / max pass drains
-    return cuda_status(launch_maybe_pdl(true, normalize_kernel, grid_for(normalize_kernel, n),
-                                        kThreads, 0, (cudaStream_t)stream, src, dst, n,
-                                        (const unsigned long long *)keys, alpha, beta));
+    // two launches: every block's keys, then the normalisation, whose blocks
+    // reduce them (a reset and atomics would be a third)
+    const int parts = std::min(grid_for<minmax_kernel<true>>(n / 4), ctx->key_pairs);
+    unsigned long long *keys = nullptr;
+    st = keys_at(ctx, 0, &keys);  // the workspace is used, as ever
+    if (st) return st;
+    keys = ctx->d_keys;
+    cudaStream_t s = (cudaStream_t)stream;
+    cudaError_t e = launch_maybe_pdl(true, minmax_kernel<true>, parts, kThreads, 0, s, src, n, keys);
+    if (e != cudaSuccess) return cuda_status(e);
+    return cuda_status(launch_maybe_pdl(true, normalize_kernel<false>, grid_for<normalize_kernel<false>>(n / 4),
+                                        kThreads, 0, s, src, dst, n, (const unsigned long long *)keys, parts,
+                                        alpha, beta));
 }
 
 int glsfft_fft_display(glsfft_context ctx, const float *frame, const float *window, float *dst,
@@ -464,14 +513,14 @@ int glsfft_fft_display(glsfft_context ctx, const float *frame, const float *wind
                 : launch_cols(rows, LD_C2, ST_LOGMAG_MINMAX, c, 1, s);
     } else {
         auto kern = spec_mag_kernel<true, true>;
-        kern<<<grid_for(kern, n), kThreads, 0, s>>>(spec, dst, n, offset, keys);
+        kern<<<grid_for<spec_mag_kernel<true, true>>(n), kThreads, 0, s>>>(spec, dst, n, offset, keys);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) return cuda_status(e);
     // normalize(0, 1, NORM_MINMAX) in place
-    return cuda_status(launch_maybe_pdl(true, normalize_kernel, grid_for(normalize_kernel, n),
+    return cuda_status(launch_maybe_pdl(true, normalize_kernel<true>, grid_for<normalize_kernel<true>>(n / 4),
                                         kThreads, 0, s, (const float *)dst, dst, n,
-                                        (const unsigned long long *)keys, 0.0, 1.0));
+                                        (const unsigned long long *)keys, 1, 0.0, 1.0));
 }
 
 }  // extern "C"

@@ -97,12 +97,10 @@ struct MinMaxAny {
     __device__ __forceinline__ unsigned long long kmax() const { return max_key(vmax, imax); }
 };
 
-// Block-wide max of both keys; thread 0 issues the atomics.  `red` holds
+// Block-wide max of both keys, on thread 0 (min, max).  `red` holds
 // 2 * (blockDim.x / 32) entries of shared memory.
-__device__ __forceinline__ void block_minmax_commit(unsigned long long kmin,
-                                                    unsigned long long kmax,
-                                                    unsigned long long *red,
-                                                    unsigned long long *dst2) {
+__device__ __forceinline__ ulonglong2 block_minmax(unsigned long long kmin, unsigned long long kmax,
+                                                   unsigned long long *red) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
         const unsigned long long a = __shfl_xor_sync(0xffffffffu, kmin, off);
@@ -116,14 +114,24 @@ __device__ __forceinline__ void block_minmax_commit(unsigned long long kmin,
         red[warps + warp] = kmax;
     }
     __syncthreads();
+    unsigned long long bmin = 0, bmax = 0;
     if (threadIdx.x == 0) {
-        unsigned long long bmin = 0, bmax = 0;
         for (int w = 0; w < warps; w++) {
             bmin = red[w] > bmin ? red[w] : bmin;
             bmax = red[warps + w] > bmax ? red[warps + w] : bmax;
         }
-        if (bmin) atomicMax(dst2, bmin);
-        if (bmax) atomicMax(dst2 + 1, bmax);
+    }
+    return make_ulonglong2(bmin, bmax);
+}
+// The same, and thread 0 issues the atomics.
+__device__ __forceinline__ void block_minmax_commit(unsigned long long kmin,
+                                                    unsigned long long kmax,
+                                                    unsigned long long *red,
+                                                    unsigned long long *dst2) {
+    const ulonglong2 k = block_minmax(kmin, kmax, red);
+    if (threadIdx.x == 0) {
+        if (k.x) atomicMax(dst2, k.x);
+        if (k.y) atomicMax(dst2 + 1, k.y);
     }
 }
 

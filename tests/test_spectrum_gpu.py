@@ -215,3 +215,35 @@ def test_fft_display_back_to_back_frames(ctx, torch_cuda, n):
         ctx.fft_display(f.data_ptr(), win.data_ptr(), alone.data_ptr(), n, n, 1.0, s)
         torch.cuda.synchronize()
         assert _eq(g_, alone.cpu().numpy())
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (1, 3), (5, 7), (33, 31), (1, 4099), (1081, 1919), (3000, 1411)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_normalize_after_element_ops(ctx, torch_cuda, oracle, shape, shift):
+    """The chained element kernels (each one's successor already resident) on
+    images of odd sizes, aligned and 4 bytes off alignment, with extremes in
+    the first and last element, NaN and a value beyond the literal among them:
+    magSpectrums, then normalize, bit-exact, called twice on other data."""
+    torch = torch_cuda
+    r, c = shape
+    s = stream_handle(torch)
+    for seed in (5, 6):
+        x = _c(r, c, seed) * np.float32(3)
+        x.flat[-1] = 50
+        x.flat[0] = 0
+        if r * c > 100:
+            x.flat[17] = np.nan
+            x.flat[60] = np.inf
+        d = _dev(torch, x)
+        buf = torch.empty(2 * (r * c + 8), dtype=torch.float32, device="cuda")
+        mag, view = buf[shift:shift + r * c], buf[r * c + 4 + shift:][:r * c]
+        ctx.mag_spectrums(d.data_ptr(), mag.data_ptr(), r, c, s)
+        ctx.normalize_minmax(mag.data_ptr(), view.data_ptr(), r, c, -1.0, 2.0, s)
+        ctx.normalize_minmax(mag.data_ptr(), mag.data_ptr(), r, c, -1.0, 2.0, s)
+        torch.cuda.synchronize()
+        want = oracle.normalize_minmax(oracle.mag_spectrums(x), -1.0, 2.0)
+        for got in (view, mag):
+            got = got.cpu().numpy().reshape(shape)
+            assert np.array_equal(np.isnan(got), np.isnan(want))
+            ok = ~np.isnan(want)
+            assert np.array_equal(got[ok], want[ok]), seed
