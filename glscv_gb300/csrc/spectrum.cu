@@ -186,6 +186,15 @@ __global__ void minmax_reset_kernel(unsigned long long *keys) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// 16-byte loads in flight per thread of the min / max pass
+constexpr int kMinMaxBatch = 8;
+// Its blocks: enough for every thread to fill one batch, or two per SM while
+// that is fewer (a thread runs its whole batch, so a grid of one load per
+// thread spent seven of eight slots on nothing: 1081 x 1919 with
+// normalisation 10.2 us, 7.0 with this).
+template <bool PARTIAL>
+int minmax_grid(size_t n);
+
 // PARTIAL = false: after minmax_reset_kernel, the keys are reduced over the
 // grid by atomics.  The input was complete before the reset kernel started
 // (stream order); only the keys come from it, so the pass waits for its
@@ -211,7 +220,7 @@ __global__ void __launch_bounds__(kThreads) minmax_kernel(const float *__restric
         // the visiting order per thread stays increasing).  The last batch is
         // predicated, its missing slots NaN, which never compares, so the
         // ragged end costs one round trip rather than one per load.
-        constexpr int kBatch = 8;
+        constexpr int kBatch = kMinMaxBatch;
         const float4 none = make_float4(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff),
                                         __int_as_float(0x7fffffff), __int_as_float(0x7fffffff));
         for (size_t i = tid; i < nv; i += kBatch * stride) {
@@ -251,7 +260,7 @@ __global__ void __launch_bounds__(kThreads) normalize_kernel(const float *x, flo
                                                              const unsigned long long *keys,
                                                              int parts, double alpha, double beta) {
     __shared__ unsigned long long red[2 * (kThreads / 32)];
-    __shared__ ulonglong2 s_key;
+    __shared__ float2 s_lin;
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const bool vec = al16(x) && al16(d);
@@ -276,14 +285,19 @@ __global__ void __launch_bounds__(kThreads) normalize_kernel(const float *x, flo
     }
     if (parts > 1) {
         const ulonglong2 k = block_minmax(kmin, kmax, red);
-        if (threadIdx.x == 0) s_key = k;
-    } else if (threadIdx.x == 0) {
-        s_key = make_ulonglong2(kmin, kmax);
+        kmin = k.x;
+        kmax = k.y;
+    }
+    // one thread runs the FP64 steps: GB300's FP64 pipe takes 16 cycles a
+    // warp instruction, and every thread computing them cost the pass about
+    // 4 us (1081 x 1919: min / max and normalisation 11.2 -> 5.6 us)
+    if (threadIdx.x == 0) {
+        const double mn = min_key_value(kmin), mx = max_key_value(kmax);
+        const float f = __fdiv_rn((float)(beta - alpha), (float)(mx - mn));
+        s_lin = make_float2(f, (float)__dsub_rn(alpha, __dmul_rn((double)f, mn)));
     }
     __syncthreads();
-    const double mn = min_key_value(s_key.x), mx = max_key_value(s_key.y);
-    const float scl = __fdiv_rn((float)(beta - alpha), (float)(mx - mn));
-    const float c = (float)__dsub_rn(alpha, __dmul_rn((double)scl, mn));
+    const float scl = s_lin.x, c = s_lin.y;
     auto step = [&](const float4 q) {
         return make_float4(__fadd_rn(c, __fmul_rn(scl, q.x)), __fadd_rn(c, __fmul_rn(scl, q.y)),
                            __fadd_rn(c, __fmul_rn(scl, q.z)), __fadd_rn(c, __fmul_rn(scl, q.w)));
@@ -296,6 +310,13 @@ __global__ void __launch_bounds__(kThreads) normalize_kernel(const float *x, flo
         if (i < nv) fetch(i);
     }
     for (size_t i = nv * 4 + tid; i < n; i += stride) d[i] = __fadd_rn(c, __fmul_rn(scl, x[i]));
+}
+
+template <bool PARTIAL>
+int minmax_grid(size_t n) {
+    const size_t nv = (n + 3) / 4;
+    const size_t least = std::min(nv, (size_t)2 * kThreads * (size_t)std::max(sm_count(), 1));
+    return grid_for<minmax_kernel<PARTIAL>>(std::max((nv + kMinMaxBatch - 1) / kMinMaxBatch, least));
 }
 
 bool misaligned(const void *p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) != 0; }
@@ -404,7 +425,7 @@ int glsfft_min_max_loc_async(glsfft_context ctx, const float *src, int rows, int
     minmax_reset_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(d_keys);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_status(e);
-    return cuda_status(launch_maybe_pdl(true, minmax_kernel<false>, grid_for<minmax_kernel<false>>(n / 4),
+    return cuda_status(launch_maybe_pdl(true, minmax_kernel<false>, minmax_grid<false>(n),
                                         kThreads, 0, (cudaStream_t)stream, src, n, d_keys));
 }
 
@@ -448,7 +469,7 @@ int glsfft_normalize_minmax(glsfft_context ctx, const float *src, float *dst, in
     const size_t n = (size_t)rows * cols;
     // two launches: every block's keys, then the normalisation, whose blocks
     // reduce them (a reset and atomics would be a third)
-    const int parts = std::min(grid_for<minmax_kernel<true>>(n / 4), ctx->key_pairs);
+    const int parts = std::min(minmax_grid<true>(n), ctx->key_pairs);
     unsigned long long *keys = nullptr;
     st = keys_at(ctx, 0, &keys);  // the workspace is used, as ever
     if (st) return st;
