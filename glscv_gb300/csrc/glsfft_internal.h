@@ -97,6 +97,11 @@ bool fused_applies(int rows, int cols);
 cudaError_t launch_fused(const PassArgs &a, bool real_in, float scale_cols, int images,
                          cudaStream_t s);
 
+// n floats of page-locked host memory to dst by a kernel on a few SMs
+// (frame_copy.cu).  It does not wait for its predecessor on the stream beyond
+// that one's last loads: the caller makes sure nobody else uses dst.
+cudaError_t launch_frame_copy(const float *host, float *dst, size_t n, cudaStream_t s);
+
 // The streamed column pass for 2048- and 4096-point columns (fft_stream.cu;
 // cols must be true): whether it applies to these arguments (contiguous
 // complex images, 16-byte aligned, the column count a multiple of the

@@ -52,7 +52,8 @@ enum { REQ_QUEUED = 0, REQ_RUNNING = 1, REQ_DONE = 2, REQ_FAILED = 3 };
 struct Request {
     int ref = 0;
     const float *frame = nullptr;  // host pointer, valid until completion
-    bool direct = false;           // the row kernel reads `frame` itself
+    bool direct = false;           // `frame` is device-readable (page-locked)
+    bool linked = false;           // direct, by the link stream's copy kernel
     int box = 5;
     // arrival: the scheduled arrival (latency counts from it); submitted: when
     // the request was queued; admitted: when a dispatcher took a slot and
@@ -72,6 +73,7 @@ struct Slot {
     cudaStream_t stream = nullptr;
     cudaEvent_t start = nullptr;   // recorded before the frame's copy (timing)
     cudaEvent_t copied = nullptr;  // recorded after the frame's copy (timing)
+    cudaEvent_t linked = nullptr;  // recorded after the frame's copy kernel (link stream)
     cudaEvent_t done = nullptr;   // recorded after the last launch (timing)
     double *h_result = nullptr;      // pinned and mapped, 8 doubles
     double *h_result_dev = nullptr;  // its device-side address
@@ -80,6 +82,14 @@ struct Slot {
 };
 
 constexpr int kDispatchers = 3;
+// Page-locked frames of at least this many pixels go through the link
+// stream's copy kernel while other requests wait or run.  A row kernel that
+// reads a large frame itself holds the registers of every SM for as long as
+// the link takes, and the others' column kernels wait.  Smaller frames, and a
+// request on its own, are sooner done without the extra launch and event.
+// GB300, bursts of six, read by the row kernel / copied: 2048^2 831 / 640 us,
+// 1024^2 236 / 213, 512^2 133 / 139; alone 2048^2 189 / 190.
+constexpr size_t kLinkedPixels = (size_t)1 << 20;
 
 size_t workspace_bytes(int rows, int cols) {
     const size_t n = (size_t)rows * cols;
@@ -96,6 +106,8 @@ struct glsfft_server_s {
     Arena arena;
     std::vector<Reference> refs;
     std::vector<Slot> slots;
+    cudaStream_t link = nullptr;  // large frames' copy kernels, one after another
+    std::mutex link_mu;           // a copy kernel and its event are issued together
     std::mutex mu;
     std::condition_variable cv_dispatch, cv_poll, cv_done;
     std::deque<long long> queue;
@@ -128,19 +140,27 @@ int launch_request(glsfft_server srv, const Reference &ref, const Request &rq, S
     const float *win = ref.has_window ? reinterpret_cast<const float *>(srv->d_base + ref.win_off) : nullptr;
     cudaStream_t s = slot.stream;
 
-    // five calls: the frame's upload, three launches (the POC column pass
+    // the frame's way to the device, three launches (the POC column pass
     // zeroes the argmax key; the last block of the inverse row pass computes
     // the centroid and writes it into the slot's mapped pinned buffer), the event
     cudaError_t e = cudaEventRecord(slot.start, s);
-    if (e == cudaSuccess && !rq.direct)
+    if (e == cudaSuccess && rq.linked) {
+        // the copy kernels of all requests queue on one stream, so that one
+        // at a time has the host link and the first frames arrive first
+        std::lock_guard<std::mutex> lock(srv->link_mu);
+        e = launch_frame_copy(rq.frame, frame, n, srv->link);
+        if (e == cudaSuccess) e = cudaEventRecord(slot.linked, srv->link);
+    } else if (e == cudaSuccess && !rq.direct) {
         e = cudaMemcpyAsync(frame, rq.frame, 4 * n, cudaMemcpyHostToDevice, s);
+    }
+    if (e == cudaSuccess && rq.linked) e = cudaStreamWaitEvent(s, slot.linked, 0);
     if (e == cudaSuccess) e = cudaEventRecord(slot.copied, s);
     if (e != cudaSuccess) return cuda_status(e);
     PassArgs a{};
     // direct: the windowed row pass loads the page-locked host frame over the
     // host link itself (its device address is the host address under unified
-    // addressing), so no copy-engine transfer precedes it
-    a.in0 = rq.direct ? rq.frame : frame;
+    // addressing), so no transfer precedes it
+    a.in0 = rq.direct && !rq.linked ? rq.frame : frame;
     a.out0 = f2;
     a.window = win;
     a.rows = rows;
@@ -214,6 +234,8 @@ void dispatcher_main(glsfft_server srv) {
             srv->admitted++;
             srv->peak_in_flight = std::max<long long>(srv->peak_in_flight, srv->in_flight);
             srv->peak_arena = std::max(srv->peak_arena, srv->arena.in_use());
+            rq.linked = rq.direct && (size_t)ref.rows * ref.cols >= kLinkedPixels &&
+                        (srv->in_flight > 1 || !srv->queue.empty());
             const Request snapshot = rq;
             lock.unlock();
             const int st = launch_request(srv, ref, snapshot, slot);
@@ -371,12 +393,22 @@ int glsfft_server_create(glsfft_context ctx, int slots, size_t hbm_budget, glsff
         delete srv;
         return GLSFFT_ERROR_OUT_OF_MEMORY;
     }
+    // the copy kernels' few blocks go before the waiting blocks of other grids
+    int least = 0, greatest = 0;
+    if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&srv->link, cudaStreamNonBlocking, greatest) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(srv->d_base);
+        delete srv;
+        return GLSFFT_ERROR_CUDA;
+    }
     srv->arena.reset(hbm_budget);
     srv->slots.resize(slots);
     for (auto &s : srv->slots) {
         cudaError_t e = cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreate(&s.start);
         if (e == cudaSuccess) e = cudaEventCreate(&s.copied);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s.linked, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreate(&s.done);
         if (e == cudaSuccess) e = cudaHostAlloc(&s.h_result, 8 * sizeof(double), cudaHostAllocMapped);
         if (e == cudaSuccess) e = cudaHostGetDevicePointer(&s.h_result_dev, s.h_result, 0);
@@ -386,9 +418,11 @@ int glsfft_server_create(glsfft_context ctx, int slots, size_t hbm_budget, glsff
                 if (t.stream) cudaStreamDestroy(t.stream);
                 if (t.start) cudaEventDestroy(t.start);
                 if (t.copied) cudaEventDestroy(t.copied);
+                if (t.linked) cudaEventDestroy(t.linked);
                 if (t.done) cudaEventDestroy(t.done);
                 if (t.h_result) cudaFreeHost(t.h_result);
             }
+            cudaStreamDestroy(srv->link);
             cudaFree(srv->d_base);
             delete srv;
             return GLSFFT_ERROR_CUDA;
@@ -597,8 +631,13 @@ int glsfft_server_destroy(glsfft_server srv) {
         }
         if (s.start) cudaEventDestroy(s.start);
         if (s.copied) cudaEventDestroy(s.copied);
+        if (s.linked) cudaEventDestroy(s.linked);
         if (s.done) cudaEventDestroy(s.done);
         if (s.h_result) cudaFreeHost(s.h_result);
+    }
+    if (srv->link) {
+        cudaStreamSynchronize(srv->link);
+        cudaStreamDestroy(srv->link);
     }
     if (srv->d_base) cudaFree(srv->d_base);
     delete srv;

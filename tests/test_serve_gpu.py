@@ -158,3 +158,26 @@ def test_direct_frame_read_equals_copy(ctx, torch_cuda):
         pageable = np.ascontiguousarray(frames[3][4])
         r = srv.wait(srv.submit(frames[3][0], pageable.ctypes.data))[0]
         assert r == copy[3]
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+def test_large_frames_in_a_burst(ctx, torch_cuda, offset):
+    """Large frames of a burst reach the device by the copy kernel (alone they
+    are read by the row pass): the results are the same bit for bit, from
+    16-byte aligned host memory and from 4 bytes off."""
+    torch = torch_cuda
+    n = 1024
+    with g.Server(ctx, slots=4, hbm_budget=1 << 28) as srv:
+        a = np.random.default_rng(3).uniform(0, 1, (n, n)).astype(np.float32)
+        ref = torch.from_numpy(a).cuda()
+        rid = srv.add_reference(ref.data_ptr(), None, n, n)
+        frames = []
+        for k in range(6):
+            buf = torch.empty(n * n + 4, dtype=torch.float32, pin_memory=True)
+            buf[offset:offset + n * n] = torch.from_numpy(np.roll(a, (3 * k, -5 * k), axis=(0, 1)).ravel())
+            frames.append(buf)
+        ptrs = [f.data_ptr() + 4 * offset for f in frames]
+        alone = [srv.wait(srv.submit(rid, p))[0] for p in ptrs]
+        for _ in range(3):
+            tickets = [srv.submit(rid, p) for p in ptrs]
+            assert [srv.wait(t)[0] for t in tickets] == alone
