@@ -4,8 +4,9 @@
 // kernel itself, a frame holds the registers of every SM for as long as the
 // link takes, and the column kernels of other requests (a whole SM's
 // registers each) wait; this kernel keeps the link full from a few blocks --
-// kBlocks x 512 threads x 8 loads of 16 bytes, 1.5 MB in flight against the
-// link's ~0.4 MB of bandwidth x latency -- and leaves the other SMs to them.
+// 16 x 256 threads x 8 loads of 16 bytes, 0.5 MB in flight; 8 blocks already
+// measured the link's rate, 16 MB in 86 us with 8 to 304 blocks -- and leaves
+// the other SMs to them.
 // The next frame's copy, launched as this one's programmatic dependent, may
 // start when every block has issued its last loads.
 #include <cstdint>
