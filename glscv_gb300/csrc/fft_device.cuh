@@ -187,6 +187,19 @@ template <> struct Dft<16> {
 struct SyncBlock {
     __device__ __forceinline__ void operator()() const { __syncthreads(); }
 };
+// Lines of T consecutive threads, LINES of them per block: a line's exchange
+// waits for its own warps only -- the warp itself, or a named barrier per line
+// (1 + line; 15 at most, else the whole block) -- so the lines of a block
+// drift apart and one's shared-memory traffic overlaps another's arithmetic.
+template <int T, int LINES>
+struct SyncLines {
+    __device__ __forceinline__ void operator()() const {
+        if constexpr (T <= 32) __syncwarp();
+        else if constexpr (LINES <= 15)
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + threadIdx.x / T), "n"(T) : "memory");
+        else __syncthreads();
+    }
+};
 struct SyncCompute256 {
     __device__ __forceinline__ void operator()() const {
         asm volatile("bar.sync 1, 256;" ::: "memory");
