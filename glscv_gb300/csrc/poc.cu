@@ -5,9 +5,17 @@
 
 namespace glsfft {
 
-template <int N>
+// W columns per block, or half as many while that leaves more than a third of
+// the SMs without a block (as the plain column pass, fft_cols.cu): 1024 x 512
+// 32.0 -> 28.3 us a call, 64 x 64 24.3 -> 22.2.  Not below 4 columns: 16-byte
+// pieces write half sectors (1024 x 64 complex columns 10.6 us with 4, 13.5
+// with 2).
+template <int N, int W = poc_W(N)>
 static cudaError_t poc_t(const PassArgs &a, cudaStream_t s) {
-    constexpr int E = poc_E(N), W = poc_W(N), T = poc_T(N);
+    constexpr int E = poc_E(N), T = poc_T(N);
+    if constexpr (N >= 64 && W >= 8 && W / 2 * T >= 32) {
+        if (a.spread && 3 * ((a.cols + W - 1) / W) < 2 * sm_count()) return poc_t<N, W / 2>(a, s);
+    }
     constexpr int threads = W * T;
     constexpr size_t smem = num_passes(N) > 1 ? sizeof(float2) * (size_t)padded_count(N * W) : 0;
     auto kern = poc_cols_kernel<N, E, W>;
