@@ -27,6 +27,21 @@ static cudaError_t cols_t(const PassArgs &a, int images, cudaStream_t s) {
     return cols_w<N, W, LD, ST>(a, images, s);
 }
 
+// 2048-point columns.  Up to two rounds of one 8-column block per SM take
+// that (64-byte row segments), many rounds the streamed pass, which overlaps a
+// tile's copy with the one before it; between them 4 columns, two blocks per
+// SM.  GB300, us with 4 columns / 8 / streamed: 1024 columns 12.5 / 10.6 /
+// 12.6, 2048 20.7 / 18.7 / 20.7, 4096 39.6 / 43.7 / 42.6, 9472 82 / 84 / 72.
+// All give the same bits.
+template <int LD, int ST>
+static cudaError_t cols_2048(const PassArgs &a, int images, cudaStream_t s) {
+    const long long total = (long long)a.cols * images, round = 8LL * sm_count();
+    if (a.spread && total <= 2 * round && total >= round / 2) return cols_w<2048, 8, LD, ST>(a, images, s);
+    if (a.spread && total >= 5 * round && stream_pass_applies(2048, true, a, images, ST))
+        return launch_stream_pass(2048, true, a, images, s, ST);
+    return cols_t<2048, cols_W(2048), LD, ST>(a, images, s);
+}
+
 template <int LD, int ST>
 static cudaError_t cols_n(int n, const PassArgs &a, int images, cudaStream_t s) {
     switch (n) {
@@ -41,7 +56,7 @@ static cudaError_t cols_n(int n, const PassArgs &a, int images, cudaStream_t s) 
     case 256: return cols_t<256, cols_W(256), LD, ST>(a, images, s);
     case 512: return cols_t<512, cols_W(512), LD, ST>(a, images, s);
     case 1024: return cols_t<1024, cols_W(1024), LD, ST>(a, images, s);
-    case 2048: return cols_t<2048, cols_W(2048), LD, ST>(a, images, s);
+    case 2048: return cols_2048<LD, ST>(a, images, s);
     case 4096: return cols_t<4096, cols_W(4096), LD, ST>(a, images, s);
     default: return cudaErrorInvalidValue;
     }
