@@ -308,6 +308,96 @@ struct LineFft {
         pass<0>(x, t, sm, tw);
     }
 
+    // Two lines of this thread's at once, each with an exchange buffer of its
+    // own: one set of barriers and of twiddle loads for both, and one line's
+    // shared-memory traffic beside the other's arithmetic.
+    template <class Sm, class Tw>
+    __device__ __forceinline__ static void run2(float2 (&x)[E], float2 (&y)[E], int t, Sm sx, Sm sy,
+                                                Tw tw) {
+        pass2<0>(x, y, t, sx, sy, tw);
+    }
+
+    // Multiply butterfly inputs v, u, ... (position k of a pass with radix R
+    // and span Ns) by their twiddles.  w^0..w^(R/2-1) come from the table
+    // (R/4 16-byte loads); w^(R/2+r) = w^(R/2) * w^r, one extra rounding,
+    // halves the twiddle loads (entry R/2 is stored in slot 0, whose value
+    // w^0 = 1 is never needed)
+    template <int p, int R, int Ns, class Tw, class... V>
+    __device__ __forceinline__ static void twiddle(Tw tw, int k, V &...v) {
+        auto mul = [&](int r, float2 w) { ((v[r] = cmul(v[r], w)), ...); };
+        if constexpr (R == 2) {
+            mul(1, tw_single<N, MB, p, Ns * R>(tw, k));
+        } else {
+            float2 wh = make_float2(1.f, 0.f);  // w^(R/2), from pair 0
+#pragma unroll
+            for (int h = 0; h < R / 4; h++) {
+                const float4 q = tw_pair<N, MB, p, R, Ns * R>(tw, k, h);
+                const float2 w0 = make_float2(q.x, q.y), w1 = make_float2(q.z, q.w);
+                if (h == 0) {
+                    wh = w0;
+                    mul(R / 2, wh);
+                } else {
+                    mul(2 * h, w0);
+                    mul(2 * h + R / 2, cmul(wh, w0));
+                }
+                mul(2 * h + 1, w1);
+                mul(2 * h + 1 + R / 2, cmul(wh, w1));
+            }
+        }
+    }
+
+    template <int p, class Sm, class Tw>
+    __device__ __forceinline__ static void pass2(float2 (&x)[E], float2 (&y)[E], int t, Sm sx, Sm sy,
+                                                 Tw tw) {
+        if constexpr (p < P) {
+            const Sync sync{};
+            constexpr int R = pass_radix(N, p, MB);
+            constexpr int Ns = pass_span(N, p, MB);
+            constexpr int S = E / R;
+            constexpr bool last = (Ns * R == N);
+#pragma unroll
+            for (int s = 0; s < S; s++) {
+                const int j = t + s * T;
+                float2 v[R], u[R];
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    v[r] = x[s + r * S];
+                    u[r] = y[s + r * S];
+                }
+                if constexpr (Ns > 1) twiddle<p, R, Ns>(tw, j & (Ns - 1), v, u);
+                Dft<R>::run(v);
+                const int d = (j / Ns) * Ns * R + (j & (Ns - 1));
+                if constexpr (last) {
+#pragma unroll
+                    for (int r = 0; r < R; r++) x[s + r * S] = v[r];
+                } else {
+                    float2 *o = sx.at(d);
+#pragma unroll
+                    for (int r = 0; r < R; r++) o[slot_step<Sm, Ns>(r)] = v[r];
+                }
+                Dft<R>::run(u);
+                if constexpr (last) {
+#pragma unroll
+                    for (int r = 0; r < R; r++) y[s + r * S] = u[r];
+                } else {
+                    float2 *o = sy.at(d);
+#pragma unroll
+                    for (int r = 0; r < R; r++) o[slot_step<Sm, Ns>(r)] = u[r];
+                }
+            }
+            if constexpr (!last) {
+                sync();
+                const float2 *ix = sx.at(t), *iy = sy.at(t);
+#pragma unroll
+                for (int m = 0; m < E; m++) x[m] = ix[slot_step<Sm, T>(m)];
+#pragma unroll
+                for (int m = 0; m < E; m++) y[m] = iy[slot_step<Sm, T>(m)];
+                if constexpr (p + 2 < P) sync();
+                pass2<p + 1>(x, y, t, sx, sy, tw);
+            }
+        }
+    }
+
     template <int p, class Sm, class Tw>
     __device__ __forceinline__ static void pass(float2 (&x)[E], int t, Sm sm, Tw tw) {
         if constexpr (p < P) {
@@ -323,32 +413,7 @@ struct LineFft {
                 float2 v[R];
 #pragma unroll
                 for (int r = 0; r < R; r++) v[r] = x[s + r * S];
-                if constexpr (Ns > 1) {
-                    // w^0..w^(R/2-1) come from the table (R/4 16-byte loads);
-                    // w^(R/2+r) = w^(R/2) * w^r, one extra rounding, halves
-                    // the twiddle loads (entry R/2 is stored in slot 0, whose
-                    // value w^0 = 1 is never needed)
-                    const int k = j & (Ns - 1);
-                    if constexpr (R == 2) {
-                        v[1] = cmul(v[1], tw_single<N, MB, p, Ns * R>(tw, k));
-                    } else {
-                        float2 wh = make_float2(1.f, 0.f);  // w^(R/2), from pair 0
-#pragma unroll
-                        for (int h = 0; h < R / 4; h++) {
-                            const float4 q = tw_pair<N, MB, p, R, Ns * R>(tw, k, h);
-                            const float2 w0 = make_float2(q.x, q.y), w1 = make_float2(q.z, q.w);
-                            if (h == 0) {
-                                wh = w0;
-                                v[R / 2] = cmul(v[R / 2], wh);
-                            } else {
-                                v[2 * h] = cmul(v[2 * h], w0);
-                                v[2 * h + R / 2] = cmul(v[2 * h + R / 2], cmul(wh, w0));
-                            }
-                            v[2 * h + 1] = cmul(v[2 * h + 1], w1);
-                            v[2 * h + 1 + R / 2] = cmul(v[2 * h + 1 + R / 2], cmul(wh, w1));
-                        }
-                    }
-                }
+                if constexpr (Ns > 1) twiddle<p, R, Ns>(tw, j & (Ns - 1), v);
                 Dft<R>::run(v);
                 if constexpr (last || Sm::kSplit) {
 #pragma unroll

@@ -17,7 +17,8 @@ static cudaError_t poc_t(const PassArgs &a, cudaStream_t s) {
         if (a.spread && 3 * ((a.cols + W - 1) / W) < 2 * sm_count()) return poc_t<N, W / 2>(a, s);
     }
     constexpr int threads = W * T;
-    constexpr size_t smem = num_passes(N) > 1 ? sizeof(float2) * (size_t)padded_count(N * W) : 0;
+    constexpr size_t one = num_passes(N) > 1 ? sizeof(float2) * (size_t)padded_count(N * W) : 0;
+    const size_t smem = a.flags & PF_F1_SPECTRUM ? one : 2 * one;  // an exchange buffer per spectrum
     auto kern = poc_cols_kernel<N, E, W>;
     dim3 grid((a.cols + W - 1) / W, 1);
     return launch_pass(kern, grid, threads, smem, s, a);
