@@ -313,3 +313,21 @@ def test_sync_call_graph_cache_follows_buffers(ctx, torch_cuda):
     both("A")
     (dx, dy), _ = ctx.phase_correlate(da.data_ptr(), db.data_ptr(), dw.data_ptr(), n, n, 5, s)
     assert abs(abs(dx) - 7.1) < 0.5 and abs(abs(dy) - 2.6) < 0.5
+
+
+@pytest.mark.parametrize("shape", [(64, 128), (256, 64)])
+def test_surface_does_not_depend_on_the_scale(ctx, torch_cuda, shape):
+    """The phase-only spectrum is the same whatever power of two both images
+    are multiplied by, bit for bit: the squares of the cross spectrum lie
+    inside, across and outside the range of the shared-reciprocal form."""
+    torch = torch_cuda
+    r, c = shape
+    rng = np.random.default_rng(8)
+    a = rng.uniform(-0.5, 0.5, shape).astype(np.float32)
+    b = (np.roll(a, (5, -9), axis=(0, 1)) + rng.normal(0, 0.05, shape)).astype(np.float32)
+    want = gpu_phase_correlate(ctx, torch, a, b, None, 5, want_surface=True)
+    for k in (-30, -28, -20, 20, 24):
+        f = np.float32(2.0 ** k)
+        got = gpu_phase_correlate(ctx, torch, a * f, b * f, None, 5, want_surface=True)
+        assert got[:2] == want[:2], k
+        assert np.array_equal(got[2].view(np.uint32), want[2].view(np.uint32)), k
