@@ -278,7 +278,7 @@ int glsfft::fft2d_launch(glsfft_context ctx, const void *src, void *dst, int row
 int glsfft::poc_launch(const float2 *tw, const float *src1, const float *src2,
                        const float *window, int rows, int cols, int box, float2 *f1, float2 *f2,
                        float *surface, unsigned long long *key, double *d_result,
-                       cudaStream_t s, unsigned long long *done_flag) {
+                       cudaStream_t s, unsigned long long *done_flag, int *err) {
     // three launches: rows of both images; fused POC columns (which also
     // zero the argmax key and block counter); inverse rows with the argmax
     // and, in the last block, the centroid.  All three use programmatic
@@ -307,6 +307,7 @@ int glsfft::poc_launch(const float2 *tw, const float *src1, const float *src2,
     b.scale = 1.0f;
     b.key = key;
     b.tw = tw;
+    b.err = err;
     b.pdl = b.spread = 1;
     e = launch_poc_cols(rows, b, s);
     if (e != cudaSuccess) return cuda_status(e);
@@ -593,7 +594,7 @@ int glsfft_phase_correlate_async(glsfft_context ctx, const float *src1, const fl
     ctx->surface = surface;
     ctx->surface_count = n;
     return poc_launch(ctx->d_tw, src1, src2, window, rows, cols, box, f1, f2, surface, key,
-                      d_result, (cudaStream_t)stream);
+                      d_result, (cudaStream_t)stream, nullptr, ctx->d_status);
 }
 
 // The synchronous call's three launches into the context's mapped result.
@@ -628,7 +629,7 @@ static int poc_sync_launch(glsfft_context ctx, const float *src1, const float *s
         if (pg.exec) cudaGraphExecDestroy(pg.exec);
         pg = {src1, src2, window, rows, cols, box, ctx->ws, nullptr};
         return poc_launch(ctx->d_tw, src1, src2, window, rows, cols, box, f1, f2, surface, key,
-                          ctx->h_result_dev, s, flag);
+                          ctx->h_result_dev, s, flag, ctx->d_status);
     }
     if (!pg.exec) {  // the first repeat
         if (!ctx->capture_stream &&
@@ -639,7 +640,7 @@ static int poc_sync_launch(glsfft_context ctx, const float *src1, const float *s
                 cudaSuccess) {
             cudaGraph_t graph = nullptr;
             st = poc_launch(ctx->d_tw, src1, src2, window, rows, cols, box, f1, f2, surface, key,
-                            ctx->h_result_dev, ctx->capture_stream, flag);
+                            ctx->h_result_dev, ctx->capture_stream, flag, ctx->d_status);
             const cudaError_t e = cudaStreamEndCapture(ctx->capture_stream, &graph);
             if (st || e != cudaSuccess || !graph ||
                 cudaGraphInstantiate(&pg.exec, graph, 0) != cudaSuccess)
@@ -650,7 +651,7 @@ static int poc_sync_launch(glsfft_context ctx, const float *src1, const float *s
     }
     if (pg.exec) return cuda_status(cudaGraphLaunch(pg.exec, s));
     return poc_launch(ctx->d_tw, src1, src2, window, rows, cols, box, f1, f2, surface, key,
-                      ctx->h_result_dev, s, flag);
+                      ctx->h_result_dev, s, flag, ctx->d_status);
 }
 
 int glsfft_phase_correlate(glsfft_context ctx, const float *src1, const float *src2,

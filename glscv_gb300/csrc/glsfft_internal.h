@@ -102,6 +102,12 @@ cudaError_t launch_fused(const PassArgs &a, bool real_in, float scale_cols, int 
 // that one's last loads: the caller makes sure nobody else uses dst.
 cudaError_t launch_frame_copy(const float *host, float *dst, size_t n, cudaStream_t s);
 
+// The persistent phaseCorrelate column pass (poc_stream.cu): whether it takes
+// these arguments (1024-, 2048- or 4096-point columns, whole tiles, 16-byte
+// aligned, a status word), and its launch.
+bool poc_stream_applies(int n, const PassArgs &a);
+cudaError_t launch_poc_stream(int n, const PassArgs &a, cudaStream_t s);
+
 // The streamed column pass for 2048- and 4096-point columns (fft_stream.cu;
 // cols must be true): whether it applies to these arguments (contiguous
 // complex images, 16-byte aligned, the column count a multiple of the

@@ -178,6 +178,7 @@ int launch_request(glsfft_server srv, const Reference &ref, const Request &rq, S
     b.scale = 1.0f;
     b.flags = PF_F1_SPECTRUM;
     b.key = key;
+    b.err = srv->ctx->d_status;
     b.tw = srv->ctx->d_tw;
     b.pdl = 1;  // resident while the row pass drains
     e = launch_poc_cols(rows, b, s);

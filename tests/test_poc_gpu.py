@@ -331,3 +331,26 @@ def test_surface_does_not_depend_on_the_scale(ctx, torch_cuda, shape):
         got = gpu_phase_correlate(ctx, torch, a * f, b * f, None, 5, want_surface=True)
         assert got[:2] == want[:2], k
         assert np.array_equal(got[2].view(np.uint32), want[2].view(np.uint32)), k
+
+
+@pytest.mark.parametrize("shape", [(1024, 2048), (1024, 4096), (2048, 1024), (4096, 512), (4096, 2048)])
+def test_persistent_column_pass_against_fp64(ctx, torch_cuda, oracle, shape):
+    """Shapes with more column tiles than SMs (the persistent column pass, the
+    last round partly empty): the whole surface against FP64.  White images:
+    three FP32 transforms of about 2e-7 each, whose error the phase
+    normalisation amplifies by 1 / |F| -- for a Rayleigh-distributed |F|
+    sqrt(E[1 / |F|^2]) over 2^22 bins is below 6 -- bound the relative 2-norm
+    by 5e-6.  Called twice: the second call's copies follow the first's stores."""
+    torch = torch_cuda
+    r, c = shape
+    rng = np.random.default_rng(r + c)
+    a = rng.uniform(0, 1, shape).astype(np.float32)
+    b = (np.roll(a, (-33, 71), axis=(0, 1)) + rng.normal(0, 0.05, shape)).astype(np.float32)
+    got = [gpu_phase_correlate(ctx, torch, a, b, None, 5, want_surface=True) for _ in range(2)]
+    t = np.fft.fft2(a.astype(np.float64)) * np.conj(np.fft.fft2(b.astype(np.float64)))
+    want = np.fft.fftshift(np.real(np.fft.ifft2(t / np.abs(t)))) * (r * c)
+    for (dx, dy), resp, surf in got:
+        assert np.linalg.norm(surf - want) <= 5e-6 * np.linalg.norm(want)
+        assert np.unravel_index(int(surf.argmax()), shape) == np.unravel_index(int(want.argmax()), shape)
+    assert np.array_equal(got[0][2].view(np.uint32), got[1][2].view(np.uint32))
+    assert ctx.device_status() == 0
