@@ -597,14 +597,16 @@ int glsfft_phase_correlate_async(glsfft_context ctx, const float *src1, const fl
                       d_result, (cudaStream_t)stream, nullptr, ctx->d_status);
 }
 
-// The synchronous call's three launches into the context's mapped result.
-// A call that repeats the last one's buffers, shape and workspace replays
-// them as one CUDA graph, captured at the first repeat on the context's
-// private stream (if the capture is refused, the launches themselves).  A
-// call with other buffers -- the frames of a video loop alternate -- makes
-// the three launches directly: capturing and instantiating a graph for each
-// such call cost more host time than the pipeline takes (GB300, 1024^2 with
-// changing buffers: 60 us per call with the capture, 33 us without).
+// The synchronous call's three launches into the context's mapped result.  A
+// program that keeps calling with the same buffers, shape and workspace gets
+// them as one CUDA graph, captured at its kPocGraphAfter-th call in a row on
+// the context's private stream (if the capture is refused, the launches
+// themselves): capturing and instantiating costs about 30 us of host time once,
+// a replay saves 2.2 us against the launches (GB300), so it pays after about
+// fifteen calls.  Every other call -- the frames of a video loop alternate --
+// makes the three launches (1024^2 with changing buffers: 60 us per call with
+// a capture each, 36 us without).
+constexpr int kPocGraphAfter = 16;
 static int poc_sync_launch(glsfft_context ctx, const float *src1, const float *src2,
                            const float *window, int rows, int cols, int box, cudaStream_t s) {
     const size_t n = (size_t)rows * cols;
@@ -627,11 +629,11 @@ static int poc_sync_launch(glsfft_context ctx, const float *src1, const float *s
     };
     if (!same()) {
         if (pg.exec) cudaGraphExecDestroy(pg.exec);
-        pg = {src1, src2, window, rows, cols, box, ctx->ws, nullptr};
+        pg = {src1, src2, window, rows, cols, box, ctx->ws, nullptr, 0};
         return poc_launch(ctx->d_tw, src1, src2, window, rows, cols, box, f1, f2, surface, key,
                           ctx->h_result_dev, s, flag, ctx->d_status);
     }
-    if (!pg.exec) {  // the first repeat
+    if (!pg.exec && pg.repeats < kPocGraphAfter && ++pg.repeats == kPocGraphAfter) {
         if (!ctx->capture_stream &&
             cudaStreamCreateWithFlags(&ctx->capture_stream, cudaStreamNonBlocking) != cudaSuccess)
             ctx->capture_stream = nullptr;

@@ -38,12 +38,13 @@ struct glsfft_context_s {
     // the reference-arithmetic mode's twiddle tables, per line length
     std::map<int, float2 *> exact_tw;
     // the last glsfft_phase_correlate call's buffers, shape and workspace,
-    // and, once a call has repeated them, its three launches as a CUDA graph
+    // and, once calls keep repeating them, the three launches as a CUDA graph
     struct PocGraph {
         const float *src1 = nullptr, *src2 = nullptr, *window = nullptr;
         int rows = 0, cols = 0, box = 0;
         const void *ws = nullptr;
         cudaGraphExec_t exec = nullptr;
+        int repeats = 0;  // calls in a row that repeated them
     } poc_graph;
     cudaStream_t capture_stream = nullptr;  // private stream the graph is captured on
 };

@@ -453,10 +453,10 @@ GLSFFT_API int glsfft_batch_destroy(glsfft_batch plan);
  * kernels have finished with the inputs and the workspace (the last one's
  * exit may trail by microseconds); a failed kernel is reported through the
  * stream's synchronisation.  Uses the context workspace
- * (20 * rows * cols bytes).  A call that repeats the last call's src1, src2,
- * window, shape, box and workspace (the buffers' contents may change) replays
- * the three launches as one CUDA graph, captured at the first such repeat; any
- * other call launches them directly.  Not to be called from inside a stream
+ * (20 * rows * cols bytes).  Calls that keep repeating the last call's src1,
+ * src2, window, shape, box and workspace (the buffers' contents may change)
+ * come to replay the three launches as one CUDA graph; any other call launches
+ * them directly.  Not to be called from inside a stream
  * capture.
  */
 GLSFFT_API int glsfft_phase_correlate(glsfft_context ctx, const float *src1, const float *src2,
