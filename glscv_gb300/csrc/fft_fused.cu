@@ -14,11 +14,12 @@
 // the chain load - line - turn - line - store.  Measured on GB300, 64 x 64
 // forward + inverse, calls back to back: 9.9 us in four pass launches, 7.6
 // us in two of these with 16 values a thread, 6.9 with 8.  Images of up to
-// 65,536 pixels
-// as a cluster of such blocks that exchange the columns through distributed
-// shared memory were built too: no faster than two pass launches (128 x 128
-// 5.5 against 5.0 us, 40 images of 256 x 256 13.2 against 13.3), so larger
-// images take the pass kernels.
+// 65,536 pixels as a cluster of such blocks that exchange the columns through
+// distributed shared memory were built too: no faster than two pass launches
+// (128 x 128 5.5 against 5.0 us, 40 images of 256 x 256 13.2 against 13.3), so
+// larger images take the pass kernels.
+#include <type_traits>
+
 #include "fft_config.h"
 #include "fft_kernels.cuh"
 #include "glsfft_internal.h"
@@ -29,10 +30,15 @@ namespace {
 
 constexpr int kFusedPx = 4096;  // pixels per image at most
 
-// One buffer serves the row exchange, the turned image and the column
-// exchange in turn; each use starts behind a barrier.
+// With 8 values per thread two buffers: the exchanges of the rows (inside one
+// warp each) and of the columns go through the first, the turned image through
+// the second, so the block meets at two barriers only (64 x 64: 3.51 -> 3.26
+// us a call).  With 16 values one buffer serves all three in turn, each use
+// behind a barrier (256 x 16: 4.9 us, with two buffers 5.7).
+__host__ __device__ constexpr bool fused_two(int e) { return e == 8; }
 template <int N, int E, int LD>
-__device__ __forceinline__ void fused_rows(const PassArgs &a, const void *in, float2 *buf, float2 (&x)[E]) {
+__device__ __forceinline__ void fused_rows(const PassArgs &a, const void *in, float2 *xch, float2 *turned,
+                                           float2 (&x)[E]) {
     constexpr int T = N / E;
     const int l = threadIdx.x / T, t = threadIdx.x % T;
     const bool active = l < a.rows;
@@ -40,9 +46,10 @@ __device__ __forceinline__ void fused_rows(const PassArgs &a, const void *in, fl
     for (int m = 0; m < E; m++)
         x[m] = active ? load_elem<LD>(in, nullptr, (size_t)l * N + t + m * T) : make_float2(0.f, 0.f);
     conj_line(x, a.flags & PF_CONJ_IN);
-    LineFft<N, E>::run(x, t, RowSm{buf + l * padded_count(N)}, a.tw);
+    using Sync = std::conditional_t<fused_two(E), SyncLines<T, 1>, SyncBlock>;
+    LineFft<N, E, Sync>::run(x, t, RowSm{xch + l * padded_count(N)}, a.tw);
     finish_line(x, a.scale, false);
-    __syncthreads();
+    if constexpr (!fused_two(E)) __syncthreads();
     if (active) {
         // row l of the image, in the column lines' [position][column] order:
         // kFusedPx / rows columns (those past the image are never read)
@@ -51,23 +58,23 @@ __device__ __forceinline__ void fused_rows(const PassArgs &a, const void *in, fl
 #pragma unroll
         for (int m = 0; m < E; m++) {
             const int i = (l << lw) + ((t + m * T + sh) & (N - 1));
-            buf[i + (i >> 4)] = x[m];
+            turned[i + (i >> 4)] = x[m];
         }
     }
     __syncthreads();
 }
 
 template <int N, int E>
-__device__ __forceinline__ void fused_cols(const PassArgs &a, float scale, float2 *out, float2 *buf,
-                                           float2 (&x)[E]) {
+__device__ __forceinline__ void fused_cols(const PassArgs &a, float scale, float2 *out, float2 *xch,
+                                           const float2 *turned, float2 (&x)[E]) {
     constexpr int T = N / E, W = kFusedPx / N;
     const int c = threadIdx.x % W, t = threadIdx.x / W;
     const bool active = c < a.cols;
-    const float2 *p = ColSm<W>{buf, c}.at(t);
+    const float2 *p = ColSm<W>{const_cast<float2 *>(turned), c}.at(t);
 #pragma unroll
     for (int m = 0; m < E; m++) x[m] = active ? p[slot_step<ColSm<W>, T>(m)] : make_float2(0.f, 0.f);
-    __syncthreads();
-    LineFft<N, E>::run(x, t, ColSm<W>{buf, c}, a.tw);
+    if constexpr (!fused_two(E)) __syncthreads();
+    LineFft<N, E>::run(x, t, ColSm<W>{xch, c}, a.tw);
     finish_line(x, scale, a.flags & PF_CONJ_OUT);
     if (active) store_line<N, E, T>(out + c, (size_t)a.cols, x, t, a.flags & PF_SHIFT_ROWS);
 }
@@ -75,37 +82,41 @@ __device__ __forceinline__ void fused_cols(const PassArgs &a, float scale, float
 template <int E, int LD>
 __global__ void __launch_bounds__(kFusedPx / E) fft2d_fused_kernel(const PassArgs a, float scale_cols) {
     extern __shared__ float4 smem_raw[];
-    float2 *buf = reinterpret_cast<float2 *>(smem_raw);
+    float2 *xch = reinterpret_cast<float2 *>(smem_raw), *turned = fused_two(E) ? xch + padded_count(kFusedPx) : xch;
     pdl_enter();
     const void *in = image_in(a, blockIdx.x);
     float2 *out = static_cast<float2 *>(image_out(a, blockIdx.x));
     float2 x[E];
     if constexpr (E == 8) {
-        if (a.cols == 32) fused_rows<32, E, LD>(a, in, buf, x);
-        else fused_rows<64, E, LD>(a, in, buf, x);
-        if (a.rows == 32) fused_cols<32, E>(a, scale_cols, out, buf, x);
-        else fused_cols<64, E>(a, scale_cols, out, buf, x);
+        if (a.cols == 32) fused_rows<32, E, LD>(a, in, xch, turned, x);
+        else fused_rows<64, E, LD>(a, in, xch, turned, x);
+        if (a.rows == 32) fused_cols<32, E>(a, scale_cols, out, xch, turned, x);
+        else fused_cols<64, E>(a, scale_cols, out, xch, turned, x);
     } else {
         switch (a.cols) {
-        case 16: fused_rows<16, E, LD>(a, in, buf, x); break;
-        case 32: fused_rows<32, E, LD>(a, in, buf, x); break;
-        case 64: fused_rows<64, E, LD>(a, in, buf, x); break;
-        case 128: fused_rows<128, E, LD>(a, in, buf, x); break;
-        default: fused_rows<256, E, LD>(a, in, buf, x); break;
+        case 16: fused_rows<16, E, LD>(a, in, xch, turned, x); break;
+        case 32: fused_rows<32, E, LD>(a, in, xch, turned, x); break;
+        case 64: fused_rows<64, E, LD>(a, in, xch, turned, x); break;
+        case 128: fused_rows<128, E, LD>(a, in, xch, turned, x); break;
+        default: fused_rows<256, E, LD>(a, in, xch, turned, x); break;
         }
         switch (a.rows) {
-        case 16: fused_cols<16, E>(a, scale_cols, out, buf, x); break;
-        case 32: fused_cols<32, E>(a, scale_cols, out, buf, x); break;
-        case 64: fused_cols<64, E>(a, scale_cols, out, buf, x); break;
-        case 128: fused_cols<128, E>(a, scale_cols, out, buf, x); break;
-        default: fused_cols<256, E>(a, scale_cols, out, buf, x); break;
+        case 16: fused_cols<16, E>(a, scale_cols, out, xch, turned, x); break;
+        case 32: fused_cols<32, E>(a, scale_cols, out, xch, turned, x); break;
+        case 64: fused_cols<64, E>(a, scale_cols, out, xch, turned, x); break;
+        case 128: fused_cols<128, E>(a, scale_cols, out, xch, turned, x); break;
+        default: fused_cols<256, E>(a, scale_cols, out, xch, turned, x); break;
         }
     }
 }
 
 template <int E, int LD>
 cudaError_t fused_launch(const PassArgs &a, float scale_cols, int images, cudaStream_t s) {
-    constexpr size_t smem = sizeof(float2) * (size_t)padded_count(kFusedPx);
+    constexpr size_t smem = (fused_two(E) ? 2 : 1) * sizeof(float2) * (size_t)padded_count(kFusedPx);
+    if constexpr (smem > 48 * 1024) {
+        const cudaError_t e = smem_opt_in(reinterpret_cast<const void *>(fft2d_fused_kernel<E, LD>), smem);
+        if (e != cudaSuccess) return e;
+    }
     return launch_maybe_pdl(true, fft2d_fused_kernel<E, LD>, dim3(images), dim3(kFusedPx / E), smem, s,
                             a, scale_cols);
 }
