@@ -15,9 +15,8 @@ constexpr PassShape rows_fixed_shape() {
 
 // Rows per block.  Grids of many blocks take the fixed shape's; a grid that
 // would leave SMs idle or unevenly loaded takes the SMs' even share of its
-// rows instead, in one block per SM where that fits 512 threads: 1024 rows
-// are 147 blocks of 7 (one per SM), where 256 blocks of 4 load some SMs with
-// 8 rows, and 512 rows of 512 points 128 blocks of 4 rather than 64 of 8.
+// rows instead, in one block per SM where that fits 512 threads: 512 rows of
+// 512 points are 128 blocks of 4 rather than 64 of 8.
 // Whole warps only.
 static int row_lines(int fixed, int threads_per_line, int max_lines, long long total) {
     const int sms = sm_count();
@@ -32,6 +31,21 @@ static int row_lines(int fixed, int threads_per_line, int max_lines, long long t
 
 template <int N, int LD, int ST>
 static cudaError_t rows_t(const PassArgs &a, int images, cudaStream_t s) {
+    // Up to eight 1024- or 2048-point rows per SM: blocks of 128 threads with 16
+    // values each, two rows or one.  GB300, CV_32FC1 512 x 2048 8.74 -> 8.20
+    // us, phaseCorrelate 128 x 2048 23.5 -> 21.2 (from blocks of 4 and 1 rows
+    // with 32 values a thread); 512 x 1024 forward + inverse 12.18 -> 11.82.
+    // At 4096 points 32 values stay the better (28.5 us against 29.4 on 512
+    // rows), at 512 points the even share (1024 rows 11.97 against 12.23).
+    if constexpr (N == 1024 || (N == 2048 && !(LD == LD_C2 && ST == ST_C2))) {
+        const long long total = (long long)a.rows * images, sms = sm_count();
+        if (a.spread && total <= 8 * sms && (N == 2048 || total > sms)) {
+            constexpr int LINES = 2048 / N;
+            const size_t smem = sizeof(float2) * (size_t)LINES * padded_count(N);
+            return launch_pass(fft_rows_kernel<N, 16, LINES, LD, ST>, dim3((a.rows + LINES - 1) / LINES, images),
+                               LINES * (N / 16), smem, s, a);
+        }
+    }
     constexpr PassShape sh = rows_fixed_shape<N, LD, ST>();
     constexpr int E = sh.E, T = N / E, MAXL = cmax(sh.G, 512 / T);
     const int lines = a.spread ? row_lines(sh.G, T, MAXL, (long long)a.rows * images) : sh.G;

@@ -20,13 +20,15 @@ struct FftSchedule {
 inline long long sched_key(int rows, int cols) { return ((long long)rows << 20) | cols; }
 
 // The schedules an image size runs until it is set or tuned otherwise,
-// from measurements on GB300 (one 4096^2 image, per pass): schedule 2 for
-// 2048- and 4096-point rows (4096: 61 us vs 69 us for schedule 0) and the
-// streamed pass for 4096-point columns (85 us vs 97 us); other lengths run
-// schedule 0.
+// from measurements on GB300: schedule 2 for 2048- and 4096-point rows (one
+// 4096^2 image, per pass: 45 us, as schedule 0, and ahead of it on fewer rows),
+// schedule 3 for up to 1024 2048-point rows (1024 x 2048 forward + inverse
+// 27.5 us against 29.3), and the streamed pass for 4096-point columns (68 us
+// against 91); other lengths run schedule 0.
 inline FftSchedule default_schedule(int rows, int cols) {
     FftSchedule s{};
     if (cols == 2048 || cols == 4096) s.row = 2;
+    if (cols == 2048 && rows <= 1024) s.row = 3;
     if (rows == 4096) s.col = kSchedStreamed;
     return s;
 }

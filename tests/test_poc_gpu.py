@@ -375,3 +375,30 @@ def test_sync_call_repeated_past_the_graph(native, torch_cuda):
             c2.phase_correlate_async(da.data_ptr(), buf.data_ptr(), None, n, n, box, res.data_ptr(), s)
             torch.cuda.synchronize()
             assert [dx, dy, resp] == res.cpu().numpy()[:3].tolist(), k
+
+
+@pytest.mark.parametrize("shape", [(512, 2048), (512, 1024), (256, 1024), (128, 2048), (512, 512)])
+def test_spread_launches_in_a_fresh_process(native, torch_cuda, shape):
+    """Grids of one to eight blocks per SM, each as the first call of a process
+    (the launches raise their shared memory to spread the blocks, and what one
+    call opted a kernel into would hide a missing opt-in of the next): the
+    transform, the real transform, phaseCorrelate and the display."""
+    import subprocess
+    import sys
+    rows, cols = shape
+    code = (
+        "import torch, glscv_gb300 as g\n"
+        f"r, c = {rows}, {cols}\n"
+        "ctx, s = g.Context(0), torch.cuda.current_stream().cuda_stream\n"
+        "p, d = torch.rand(r, c, device='cuda'), torch.empty(r, c, device='cuda')\n"
+        "y = torch.empty(r, c, 2, device='cuda')\n"
+        "(dx, dy), resp = ctx.phase_correlate(p.data_ptr(), p.data_ptr(), None, r, c, 5, s)\n"
+        "assert abs(dx) < 1e-3 and abs(dy) < 1e-3 and abs(resp - 1) < 1e-3\n"
+        "ctx.fft2d(p.data_ptr(), y.data_ptr(), r, c, 0, s, real_input=True)\n"
+        "ctx.fft2d(y.data_ptr(), y.data_ptr(), r, c, 3, s)\n"
+        "ctx.fft_display(p.data_ptr(), None, d.data_ptr(), r, c, 1.0, s)\n"
+        "torch.cuda.synchronize()\n"
+        "assert torch.allclose(y[..., 0], p, atol=1e-5)\n")
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120,
+                          cwd=str(g.PKG.parent))
+    assert done.returncode == 0, done.stderr[-800:]
