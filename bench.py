@@ -836,7 +836,7 @@ def run_own(args) -> None:
     plan = g.Batch(ctx, ptr_in, ptr_out, [(ROWS, COLS)] * B, (0, INV | SCALE))
     tune = None
     if args.schedule:
-        v, c, ah, lg = (int(x) for x in args.schedule.split(","))
+        v, c, ah, lg = (float(x) for x in args.schedule.split(","))
         plan.set_variant(v)
         plan.set_schedule(c, ah, lg * plan.info()["grid"])
         tune = {"fixed": plan.schedule()}
@@ -1005,10 +1005,10 @@ def run_own(args) -> None:
     peak, peak_kind = measured_peaks()
     sched = plan.schedule()
     kname = VARIANT_KERNELS[sched["variant"]]
-    lag_grids = round(sched["lag_items"] / max(1, plan.info()["grid"]))
-    kernel_name = f"{kname} 1024x1024 x{B} fwd+inv, lag {lag_grids} grids"
+    lag_grids = round(sched["lag_items"] / max(1, plan.info()["grid"]), 2)
+    kernel_name = f"{kname} 1024x1024 x{B} fwd+inv, lag {lag_grids:g} grids"
     # DRAM traffic depends on the item-order lag (L2 reuse between passes)
-    traffic = traffic_per_launch(f"{kname}x{B} lag{lag_grids}")
+    traffic = traffic_per_launch(f"{kname}x{B} lag{lag_grids:g}")
 
     # the same batch through the two-launch batched path and through the
     # plain per-image path (the >= 3x comparison)

@@ -61,14 +61,21 @@ struct glsfft_batch_s {
 namespace {
 
 // Default schedule: three warp-specialised blocks per SM, items claimed one
-// at a time, an image's next pass listed five resident grids after its
-// previous one -- the fastest schedule measured on GB300 for 64 x 1024^2
-// forward + inverse (lag 4 is 0.5 % slower there and 2 % faster on 512
-// uneven images, a difference the autotuner's 1 % keep margin lets it
-// take), 7 % faster than two items per claim at a lag of eight grids
-// (glsfft_batch_set_schedule / the autotuner can change all).
+// at a time, an image's next pass listed four and a half resident grids
+// after its previous one.  A longer lag gives a pass more time to finish
+// before its successor is claimed; a shorter one keeps more of the
+// intermediates in L2.  Measured on GB300, us per forward + inverse at lags
+// of 3.5 / 4.5 / 5 grids: 64 x 1024^2 607.6 / 607.7 / 608.7, 128 x 512^2
+// 311.5 / 305.8 / 312.7, 512 x 256^2 250.8 / 244.6 / 251.9, 128 x 64x2048
+// 143.8 / 137.2 / 138.6, 512 mixed sizes 1384 / 1390 / 1432; forward only,
+// 160 mixed 233.5 / 236.2 / 246.3.  4.5 is the largest step down from 5
+// that slowed none of the mixes tried.  Two items per claim at a lag of
+// eight grids is 7 % slower (glsfft_batch_set_schedule / the autotuner can
+// change all).
 constexpr int kDefaultClaimChunk = 1;
-constexpr int kDefaultLagGrids = 5;
+int default_lag(int grid) { return grid * 9 / 2; }
+// the default lag among lags given in whole grids (autotuner, plan cache)
+constexpr int kBuiltinLag = -1;
 
 int row_tiles_of(int rows, int cols) {
     const int lines = kBatchTileElems / cols;
@@ -263,7 +270,7 @@ int glsfft_batch_create(glsfft_context ctx, int count, const void *const *srcs,
         plan->grid = grid_for(ctx->device, plan->variant);
         if (plan->grid <= 0) st = GLSFFT_ERROR_CUDA;
         std::vector<BatchItem> items;
-        plan->lag_items = kDefaultLagGrids * plan->grid;
+        plan->lag_items = default_lag(plan->grid);
         if (!st) items = order_items(plan->images, plan->passes, plan->lag_items);
         plan->n_items = (int)items.size();
         const size_t ni = plan->images.size();
@@ -364,13 +371,13 @@ int glsfft_batch_set_variant(glsfft_batch plan, int variant) {
         if (grid != plan->grid) {
             // the item order's lag follows the resident grid
             std::vector<BatchItem> items =
-                order_items(plan->images, plan->passes, kDefaultLagGrids * grid);
+                order_items(plan->images, plan->passes, default_lag(grid));
             cudaError_t e = cudaMemcpy(static_cast<char *>(plan->d_mem) + plan->o_items,
                                        items.data(), sizeof(BatchItem) * items.size(),
                                        cudaMemcpyHostToDevice);
             if (e != cudaSuccess) return cuda_status(e);
             plan->grid = grid;
-            plan->lag_items = kDefaultLagGrids * grid;
+            plan->lag_items = default_lag(grid);
         }
     }
     plan->variant = variant;
@@ -515,9 +522,13 @@ int glsfft_batch_autotune(glsfft_batch plan, const char *cache_path, int reps, v
     key.push_back({"others", plan_cache::quote(histogram(other_sizes))});
     key.push_back({"flags", plan_cache::quote(flags)});
 
+    // a lag in resident grids; kBuiltinLag stands for default_lag
+    auto lag_of = [](int lag_grids, int grid) {
+        return lag_grids == kBuiltinLag ? default_lag(grid) : lag_grids * grid;
+    };
     auto apply = [&](int variant, int chunk, int ahead, int lag_grids) {
         int r = glsfft_batch_set_variant(plan, variant);
-        if (!r) r = glsfft_batch_set_schedule(plan, chunk, ahead, lag_grids * plan->grid);
+        if (!r) r = glsfft_batch_set_schedule(plan, chunk, ahead, lag_of(lag_grids, plan->grid));
         return r;
     };
     plan_cache::Fields hit;
@@ -526,7 +537,7 @@ int glsfft_batch_autotune(glsfft_batch plan, const char *cache_path, int reps, v
                   a = std::atoi(hit["claim_ahead"].c_str()),
                   lg = std::atoi(hit["lag_grids"].c_str());
         if (v >= BATCH_PLAIN && v <= BATCH_TMA_WS3 && c >= 1 && c <= 4 && a >= 0 && a <= 2 &&
-            lg >= 1) {
+            (lg >= 1 || lg == kBuiltinLag)) {
             st = apply(v, c, a, lg);
             if (st) return st;
             res[0] = v;
@@ -594,9 +605,23 @@ int glsfft_batch_autotune(glsfft_batch plan, const char *cache_path, int reps, v
     if (!st && shadow->n_images != plan->n_images) st = GLSFFT_ERROR_CUDA;  // routing differs
 
     // 4. every schedule: variant x item-order lag (resident grids) x claim
-    //    chunk x claim-ahead (the plain variant has no claim knobs)
+    //    chunk x claim-ahead (the plain variant has no claim knobs), and last
+    //    the default, whose lag is not a whole number of grids
     using Cand = glsfft_batch_s::Cand;
     std::vector<Cand> cands;
+    auto time_one = [&](int v, int c, int a, int lg) {
+        if (!st) st = glsfft_batch_set_variant(shadow, v);
+        if (!st) st = glsfft_batch_set_schedule(shadow, c, a, lag_of(lg, shadow->grid));
+        double m = 0.0;
+        if (!st)
+            st = time_median_ms([&]() { return glsfft_batch_execute(shadow, s); }, 2, reps, s, &m);
+        if (!st) {
+            const int dev_st = glsfft_batch_status(shadow, s);
+            if (dev_st == GLSFFT_ERROR_TIMEOUT) return;  // not a usable schedule
+            st = dev_st;
+        }
+        if (!st) cands.push_back(Cand{v, c, a, lg, m});
+    };
     const int variants[4] = {BATCH_TMA_WS2, BATCH_TMA_WS3, BATCH_TMA_WS1, BATCH_PLAIN};
     const int lags[6] = {2, 3, 4, 5, 6, 8};
     for (int v : variants) {
@@ -606,26 +631,14 @@ int glsfft_batch_autotune(glsfft_batch plan, const char *cache_path, int reps, v
                 for (int a = 0; a <= 2 && !st; a++) {
                     if (v == BATCH_PLAIN && a) continue;
                     if (a == 2 && c != 1) continue;  // deep prefetch claims one item at a time
-                    st = glsfft_batch_set_variant(shadow, v);
-                    if (!st) st = glsfft_batch_set_schedule(shadow, c, a, lg * shadow->grid);
-                    double m = 0.0;
-                    if (!st)
-                        st = time_median_ms([&]() { return glsfft_batch_execute(shadow, s); }, 2,
-                                            reps, s, &m);
-                    if (!st) {
-                        const int dev_st = glsfft_batch_status(shadow, s);
-                        if (dev_st == GLSFFT_ERROR_TIMEOUT) continue;  // not a usable schedule
-                        st = dev_st;
-                    }
-                    if (!st) cands.push_back(Cand{v, c, a, lg, m});
+                    time_one(v, c, a, lg);
                 }
             }
         }
     }
-    auto is_default = [](const Cand &c) {
-        return c.v == BATCH_TMA_WS3 && c.c == kDefaultClaimChunk && c.a == 0 &&
-               c.lg == kDefaultLagGrids;
-    };
+    const size_t swept = cands.size();
+    time_one(BATCH_TMA_WS3, kDefaultClaimChunk, 0, kBuiltinLag);
+    auto is_default = [](const Cand &c) { return c.lg == kBuiltinLag; };
     // 5. the finalists -- the six fastest of that sweep and the default --
     //    timed again in three interleaved rounds; each keeps the median of its
     //    three medians, so one noisy sample does not pick the schedule
@@ -645,7 +658,7 @@ int glsfft_batch_autotune(glsfft_batch plan, const char *cache_path, int reps, v
             for (size_t j = 0; j < finalists.size() && !st; j++) {
                 const Cand &c = cands[finalists[j]];
                 st = glsfft_batch_set_variant(shadow, c.v);
-                if (!st) st = glsfft_batch_set_schedule(shadow, c.c, c.a, c.lg * shadow->grid);
+                if (!st) st = glsfft_batch_set_schedule(shadow, c.c, c.a, lag_of(c.lg, shadow->grid));
                 double m = 0.0;
                 if (!st)
                     st = time_median_ms([&]() { return glsfft_batch_execute(shadow, s); }, 1,
@@ -667,7 +680,7 @@ int glsfft_batch_autotune(glsfft_batch plan, const char *cache_path, int reps, v
     cudaGetLastError();
     if (st) return st;
     if (cands.empty()) return GLSFFT_ERROR_TIMEOUT;
-    plan->tuned = cands;
+    plan->tuned.assign(cands.begin(), cands.begin() + swept);
 
     // 6. the fastest finalist, unless the default schedule is within the keep
     //    margin
@@ -684,7 +697,7 @@ int glsfft_batch_autotune(glsfft_batch plan, const char *cache_path, int reps, v
     res[1] = best->c;
     res[2] = best->a;
     res[3] = plan->lag_items;
-    res[5] = (int)cands.size();
+    res[5] = (int)swept;
     t[0] = best->ms;
     t[1] = def ? def->ms : 0.0;
     if (cache_path && *cache_path) {
@@ -697,7 +710,7 @@ int glsfft_batch_autotune(glsfft_batch plan, const char *cache_path, int reps, v
         key.push_back({"ms", b});
         std::snprintf(b, sizeof b, "%.6g", t[1]);
         key.push_back({"ms_default", b});
-        key.push_back({"candidates", std::to_string(cands.size())});
+        key.push_back({"candidates", std::to_string(swept)});
         if (!plan_cache::append(cache_path, key)) st = GLSFFT_ERROR_IO;
     }
     if (result) std::copy(res, res + 6, result);

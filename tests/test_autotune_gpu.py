@@ -11,6 +11,8 @@ context, so tuned schedules do not leak into other tests.
 """
 from __future__ import annotations
 
+import re
+
 import numpy as np
 import pytest
 
@@ -184,3 +186,26 @@ def test_batch_autotune_inplace_plan_untouched(tctx, torch_cuda, oracle):
         got = d_in[i].cpu().numpy()
         assert oracle.are_equal(ref, got, 64, oracle.fft_eps(max(shapes[i]), SHIFT) * 2) == 0
     b.close()
+
+
+@pytest.mark.parametrize("cached,hit", [("-1", True), ("3", True), ("0", False), ("x", False)])
+def test_cached_lag_is_in_grids_or_the_default(tctx, torch_cuda, tmp_path, cached, hit):
+    """A cached lag is a whole number of resident grids, or -1 for the
+    built-in lag of four and a half; anything else is timed again."""
+    s = stream_handle(torch_cuda)
+    cache = tmp_path / "plans.jsonl"
+    b, *_ = _plan(tctx, torch_cuda, [(64, 64)] * 3, (0,))
+    default = b.schedule()["lag_items"]
+    assert default == b.info()["grid"] * 9 // 2
+    b.autotune(str(cache), reps=1, stream=s)
+    line = re.sub(r'"lag_grids": -?\d+', f'"lag_grids": {cached}', cache.read_text())
+    line = re.sub(r'"variant": \d', '"variant": 3', line)
+    cache.write_text(line)
+    b2, *_ = _plan(tctx, torch_cuda, [(64, 64)] * 3, (0,))
+    res = b2.autotune(str(cache), reps=1, stream=s)
+    assert res["from_cache"] == hit
+    if hit:
+        want = default if cached == "-1" else int(cached) * b2.info()["grid"]
+        assert res["lag_items"] == b2.schedule()["lag_items"] == want
+    b.close()
+    b2.close()
