@@ -2,7 +2,9 @@
 // gls::fft transforms, executed as one CUDA graph.  Images the persistent
 // kernels cover (16 <= rows <= 1024, 16 <= cols <= 4096, 16-byte aligned
 // buffers) go through one persistent launch fed by a work list; any other
-// image gets its own pass launches inside the same graph.
+// image gets its own pass launches inside the same graph.  Small plans of few
+// evenly spaced runs of equal images take the batched pass launches instead
+// (direct_segments).
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -45,6 +47,18 @@ struct glsfft_batch_s {
     };
     std::vector<Other> others;  // images outside the persistent kernels' shapes
     std::vector<int> flags;
+    // the persistent images as runs of equal, evenly spaced images, when the
+    // batched pass launches are faster (direct_segments); used while the
+    // schedule is the default one
+    struct Segment {
+        const void *src;
+        void *dst;
+        int rows, cols, count;
+        size_t src_step, dst_step;
+    };
+    std::vector<Segment> segments;
+    bool pinned = false;  // a schedule was asked for: the persistent kernel it names runs
+    bool direct = false;  // the recorded graph holds the segments' launches
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     long long wait_limit_ns = 2000000000LL;
@@ -96,7 +110,118 @@ int grid_for(int device, int variant) {
     return batch_ws_grid(device, variant);  // WS1..WS3: 1..3 blocks per SM
 }
 
+// Runs of equal images at a constant, non-overlapping distance in src and in
+// dst, each a batched pass launch; empty when there are more than one per
+// graph branch or when the persistent kernel is the better one.
+//
+// A pass boundary costs a launch about 1 us and the work list, with its claim,
+// dependency poll and TMA round trips, about 5 us, so the launches win until
+// the passes no longer find the images in L2: up to 64 MiB of images (128 MiB
+// with their source).  Measured on GB300, us per execution, launches against
+// the persistent kernel: 2 x 256x512 forward 9.3 / 18.7, 16 x 256^2 12.4 /
+// 18.6, 8 x 512^2 16.5 / 27.4, 8 x 1024^2 50.3 / 54.4, there and back 2 x
+// 256x512 12.4 / 30.9, 8 x 1024^2 90.2 / 91.2; beyond: 12 x 1024^2 there and
+// back 145.5 / 143.7, 96 x 64x2048 forward 68.7 / 63.7, 256 x 256^2 88.2 /
+// 78.0.  Images of the one-launch FFT gain at any size (4000 x 64^2 forward
+// 63.6 / 86.2, there and back 123 / 157).
+//
+// Runs on parallel branches: 4 x 1024^2 in separate buffers 30.8 / 37.0, 4 x
+// 256^2 13.5 / 18.5, three mixed sizes 21.3 / 26.7; with 12 mixed sizes the
+// launches themselves take as long as the persistent kernel (42.1 / 37.7).
+constexpr size_t kDirectBytes = size_t(64) << 20;
+constexpr size_t kDirectBranches = 4;
+
+std::vector<glsfft_batch_s::Segment> direct_segments(const std::vector<BatchImage> &images) {
+    std::vector<glsfft_batch_s::Segment> segs;
+    std::map<std::pair<int, int>, size_t> last;  // the size's run that may still grow
+    size_t bytes = 0;
+    bool fused = true;
+    for (const BatchImage &im : images) {
+        const size_t img = (size_t)im.rows * im.cols * sizeof(float2);
+        fused = fused && fused_applies(im.rows, im.cols);
+        bytes += img;
+        const auto src = reinterpret_cast<uintptr_t>(im.src), dst = reinterpret_cast<uintptr_t>(im.dst);
+        auto it = last.find({im.rows, im.cols});
+        if (it != last.end()) {
+            auto &sg = segs[it->second];
+            const auto s0 = reinterpret_cast<uintptr_t>(sg.src), d0 = reinterpret_cast<uintptr_t>(sg.dst);
+            if (sg.count == 1 && src >= s0 + img && dst >= d0 + img) {
+                sg.src_step = src - s0;
+                sg.dst_step = dst - d0;
+                sg.count = 2;
+                continue;
+            }
+            if (sg.count > 1 && sg.count < kMaxBatch && src == s0 + sg.count * sg.src_step &&
+                dst == d0 + sg.count * sg.dst_step) {
+                sg.count++;
+                continue;
+            }
+        }
+        if (segs.size() == kDirectBranches) return {};
+        last[{im.rows, im.cols}] = segs.size();
+        segs.push_back({im.src, im.dst, im.rows, im.cols, 1, 0, 0});
+    }
+    if (bytes > kDirectBytes && !fused) segs.clear();
+    return segs;
+}
+
+// The launches stand in for the persistent kernel only with the context's
+// default pass schedules, which give the same bits.
+bool use_direct(glsfft_batch plan) {
+    if (plan->segments.empty() || plan->pinned || plan->args.stats) return false;
+    for (const auto &sg : plan->segments) {
+        const FftSchedule sc = schedule_for(plan->ctx->sched, sg.rows, sg.cols),
+                          d = default_schedule(sg.rows, sg.cols);
+        if (sc.row != d.row || sc.col != d.col) return false;
+    }
+    return true;
+}
+
+// The runs' pass launches, one branch of the graph each.
+int record_direct(glsfft_batch plan, cudaStream_t s) {
+    const size_t extra = plan->segments.size() - 1;
+    cudaStream_t br[kDirectBranches] = {};
+    cudaEvent_t ev[kDirectBranches] = {};
+    cudaEvent_t fork = nullptr;
+    cudaError_t e = cudaSuccess;
+    if (extra) {
+        e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventRecord(fork, s);
+    }
+    int st = GLSFFT_SUCCESS;
+    for (size_t i = 0; i <= extra && e == cudaSuccess && !st; i++) {
+        const auto &sg = plan->segments[i];
+        if (i) {
+            e = cudaStreamCreateWithFlags(&br[i], cudaStreamNonBlocking);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(br[i], fork, 0);
+            if (e != cudaSuccess) break;
+        }
+        cudaStream_t b = i ? br[i] : s;
+        const void *src = sg.src;
+        size_t step = sg.src_step;
+        for (int f : plan->flags) {
+            st = fft2d_launch(plan->ctx, src, sg.dst, sg.rows, sg.cols, f, false, b, sg.count, step,
+                              sg.dst_step);
+            if (st) break;
+            src = sg.dst;
+            step = sg.dst_step;
+        }
+        if (i && !st) e = cudaEventRecord(ev[i], b);
+    }
+    for (size_t i = 1; i <= extra && e == cudaSuccess && !st; i++) e = cudaStreamWaitEvent(s, ev[i], 0);
+    if (!st) st = cuda_status(e);
+    for (size_t i = 1; i <= extra; i++) {
+        if (ev[i]) cudaEventDestroy(ev[i]);
+        if (br[i]) cudaStreamDestroy(br[i]);
+    }
+    if (fork) cudaEventDestroy(fork);
+    return st;
+}
+
 int record(glsfft_batch plan, cudaStream_t s) {
+    plan->direct = use_direct(plan);
+    if (plan->direct) return record_direct(plan, s);
     if (plan->n_images > 0) {
         const size_t state = sizeof(unsigned) * (1 + (size_t)plan->n_images * kBatchMaxPasses) +
                              sizeof(int);
@@ -348,6 +473,7 @@ int glsfft_batch_create(glsfft_context ctx, int count, const void *const *srcs,
             a.claim_ahead = 0;
         }
     }
+    if (!st && plan->others.empty()) plan->segments = direct_segments(plan->images);
     if (!st) st = capture(plan);
     if (st) {
         if (plan->exec) cudaGraphExecDestroy(plan->exec);
@@ -381,6 +507,7 @@ int glsfft_batch_set_variant(glsfft_batch plan, int variant) {
         }
     }
     plan->variant = variant;
+    plan->pinned = true;
     return capture(plan);
 }
 
@@ -398,6 +525,7 @@ int glsfft_batch_set_schedule(glsfft_batch plan, int claim_chunk, int claim_ahea
         if (e != cudaSuccess) return cuda_status(e);
         plan->lag_items = lag_blocks;
     }
+    plan->pinned = true;
     return capture(plan);
 }
 
@@ -413,6 +541,7 @@ int glsfft_batch_status(glsfft_batch plan, void *stream) {
     if (plan->n_images == 0) return GLSFFT_SUCCESS;
     DeviceGuard g(plan->device);
     if (!g.ok()) return GLSFFT_ERROR_CUDA;
+    if (plan->direct) return cuda_status(cudaStreamSynchronize((cudaStream_t)stream));
     int err = 0;
     cudaError_t e = cudaMemcpyAsync(&err, plan->args.error, sizeof(int), cudaMemcpyDeviceToHost,
                                     (cudaStream_t)stream);
@@ -461,6 +590,7 @@ int glsfft_batch_inject_stall(glsfft_batch plan, long long wait_limit_ns) {
     // the deadline is a kernel argument baked into the graph: re-capture
     plan->wait_limit_ns = wait_limit_ns;
     plan->args.wait_limit_ns = wait_limit_ns;
+    plan->pinned = true;
     return capture(plan);
 }
 
@@ -522,14 +652,21 @@ int glsfft_batch_autotune(glsfft_batch plan, const char *cache_path, int reps, v
     key.push_back({"others", plan_cache::quote(histogram(other_sizes))});
     key.push_back({"flags", plan_cache::quote(flags)});
 
-    // a lag in resident grids; kBuiltinLag stands for default_lag
-    auto lag_of = [](int lag_grids, int grid) {
-        return lag_grids == kBuiltinLag ? default_lag(grid) : lag_grids * grid;
+    // a lag in resident grids; kBuiltinLag stands for the plan's default
+    auto set_on = [](glsfft_batch p, int variant, int chunk, int ahead, int lag_grids) {
+        const bool dflt = lag_grids == kBuiltinLag;
+        int r = glsfft_batch_set_variant(p, variant);
+        if (!r)
+            r = glsfft_batch_set_schedule(p, chunk, ahead,
+                                          dflt ? default_lag(p->grid) : lag_grids * p->grid);
+        if (!r && dflt) {
+            p->pinned = false;
+            r = capture(p);
+        }
+        return r;
     };
     auto apply = [&](int variant, int chunk, int ahead, int lag_grids) {
-        int r = glsfft_batch_set_variant(plan, variant);
-        if (!r) r = glsfft_batch_set_schedule(plan, chunk, ahead, lag_of(lag_grids, plan->grid));
-        return r;
+        return set_on(plan, variant, chunk, ahead, lag_grids);
     };
     plan_cache::Fields hit;
     if (plan_cache::lookup(cache_path, plan_cache::as_fields(key), hit)) {
@@ -603,6 +740,8 @@ int glsfft_batch_autotune(glsfft_batch plan, const char *cache_path, int reps, v
                                  scols.data(), (int)plan->flags.size(), plan->flags.data(),
                                  &shadow);
     if (!st && shadow->n_images != plan->n_images) st = GLSFFT_ERROR_CUDA;  // routing differs
+    // the plan's images may lie unevenly where the shadow's do not
+    if (!st && plan->segments.empty()) shadow->segments.clear();
 
     // 4. every schedule: variant x item-order lag (resident grids) x claim
     //    chunk x claim-ahead (the plain variant has no claim knobs), and last
@@ -610,8 +749,7 @@ int glsfft_batch_autotune(glsfft_batch plan, const char *cache_path, int reps, v
     using Cand = glsfft_batch_s::Cand;
     std::vector<Cand> cands;
     auto time_one = [&](int v, int c, int a, int lg) {
-        if (!st) st = glsfft_batch_set_variant(shadow, v);
-        if (!st) st = glsfft_batch_set_schedule(shadow, c, a, lag_of(lg, shadow->grid));
+        if (!st) st = set_on(shadow, v, c, a, lg);
         double m = 0.0;
         if (!st)
             st = time_median_ms([&]() { return glsfft_batch_execute(shadow, s); }, 2, reps, s, &m);
@@ -657,8 +795,7 @@ int glsfft_batch_autotune(glsfft_batch plan, const char *cache_path, int reps, v
         for (int r = 0; r < 3 && !st; r++) {
             for (size_t j = 0; j < finalists.size() && !st; j++) {
                 const Cand &c = cands[finalists[j]];
-                st = glsfft_batch_set_variant(shadow, c.v);
-                if (!st) st = glsfft_batch_set_schedule(shadow, c.c, c.a, lag_of(c.lg, shadow->grid));
+                st = set_on(shadow, c.v, c.c, c.a, c.lg);
                 double m = 0.0;
                 if (!st)
                     st = time_median_ms([&]() { return glsfft_batch_execute(shadow, s); }, 1,

@@ -213,12 +213,15 @@ int glsfft::ensure_workspace(glsfft_context ctx, size_t bytes) {
 // resident and waiting while the row pass drains, and the row pass of the
 // next call on the stream likewise behind this call's column pass.
 int glsfft::fft2d_launch(glsfft_context ctx, const void *src, void *dst, int rows, int cols,
-                         int flags, bool real_in, cudaStream_t s, int count) {
+                         int flags, bool real_in, cudaStream_t s, int count, size_t src_step,
+                         size_t dst_step) {
     const bool inv = flags & GLSFFT_INVERSE, scale = flags & GLSFFT_SCALE,
                shift = flags & GLSFFT_SHIFT;
     const bool do_rows = cols > 1 || rows == 1 || real_in;
     const bool do_cols = rows > 1;
     const size_t px = (size_t)rows * cols;
+    if (!src_step) src_step = px * (real_in ? sizeof(float) : sizeof(float2));
+    if (!dst_step) dst_step = px * sizeof(float2);
     const FftSchedule sc = schedule_for(ctx->sched, rows, cols);
     if (sc.row == 0 && sc.col == 0 && fused_applies(rows, cols)) {
         PassArgs a{};
@@ -230,8 +233,8 @@ int glsfft::fft2d_launch(glsfft_context ctx, const void *src, void *dst, int row
         a.flags = (inv ? PF_CONJ_IN | PF_CONJ_OUT : 0u) |
                   (shift ? PF_SHIFT_ROWS | PF_SHIFT_COLS : 0u);
         a.tw = ctx->d_tw;
-        a.in_img_bytes = px * (real_in ? sizeof(float) : sizeof(float2));
-        a.out_img_bytes = px * sizeof(float2);
+        a.in_img_bytes = src_step;
+        a.out_img_bytes = dst_step;
         return cuda_status(launch_fused(a, real_in, scale ? 1.0f / (float)rows : 1.0f, count, s));
     }
     if (do_rows) {
@@ -246,8 +249,8 @@ int glsfft::fft2d_launch(glsfft_context ctx, const void *src, void *dst, int row
         a.tw = ctx->d_tw;
         a.err = ctx->d_status;
         a.stall_ns = ctx->stall_ns;
-        a.in_img_bytes = px * (real_in ? sizeof(float) : sizeof(float2));
-        a.out_img_bytes = px * sizeof(float2);
+        a.in_img_bytes = src_step;
+        a.out_img_bytes = dst_step;
         a.pdl = a.spread = 1;
         cudaError_t e = real_in ? launch_rows(cols, LD_R1, ST_C2, a, count, s)
                                 : launch_rows_sched(cols, sc.row, a, count, s);
@@ -265,7 +268,8 @@ int glsfft::fft2d_launch(glsfft_context ctx, const void *src, void *dst, int row
         a.tw = ctx->d_tw;
         a.err = ctx->d_status;
         a.stall_ns = ctx->stall_ns;
-        a.in_img_bytes = a.out_img_bytes = px * sizeof(float2);
+        a.in_img_bytes = do_rows ? dst_step : src_step;
+        a.out_img_bytes = dst_step;
         a.pdl = a.spread = 1;
         cudaError_t e = launch_cols_sched(rows, sc.col, a, count, s);
         if (e != cudaSuccess) return cuda_status(e);

@@ -70,7 +70,8 @@ int check_fft_args(const void *src, const void *dst, int rows, int cols, int fla
 int check_poc_args(glsfft_context ctx, const float *src1, const float *src2,
                    const float *window, int rows, int cols, int box);
 int fft2d_launch(glsfft_context ctx, const void *src, void *dst, int rows, int cols, int flags,
-                 bool real_in, cudaStream_t s, int count = 1);
+                 bool real_in, cudaStream_t s, int count = 1, size_t src_step = 0,
+                 size_t dst_step = 0);  // bytes from image to image (0: contiguous images)
 // The reference-arithmetic transform (fft_exact.cu): `count` images src ->
 // dst through tmp (count * rows * cols complex, apart from src and dst).
 int fft2d_exact_launch(glsfft_context ctx, const void *src, void *dst, void *tmp, int count,

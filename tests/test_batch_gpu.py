@@ -216,3 +216,66 @@ def test_two_plans_concurrently_on_two_streams(ctx, torch_cuda):
             assert np.array_equal(d.cpu().numpy().view(np.uint32), refs[k][i].view(np.uint32)), (k, i)
     for b in plans:
         b.close()
+
+
+DIRECT_PLANS = {
+    "one image": ([(256, 512)], 0),
+    "equal images in one buffer": ([(256, 128)] * 5, 0),
+    "equal images with gaps": ([(16, 16)] * 9, 48),
+    "four runs, interleaved": ([(64, 64), (32, 2048), (1024, 64), (512, 512)] * 2, 16),
+    "two uneven sizes": ([(1024, 16), (1024, 16), (16, 4096)], 0),
+    "one run of the largest total": ([(512, 1024)] * 16, 0),
+    "just above it": ([(512, 1024)] * 17, 0),
+    "five sizes": ([(64, 64), (32, 32), (16, 64), (64, 16), (128, 32)], 0),
+}
+
+
+@pytest.mark.parametrize("name", DIRECT_PLANS)
+@pytest.mark.parametrize("flags", [(0, INV | SCALE), (SHIFT,)])
+@pytest.mark.parametrize("inplace", [False, True])
+def test_default_schedule_bit_identical_to_the_persistent_kernel(ctx, torch_cuda, name, flags,
+                                                                 inplace):
+    """The launches that small, even plans use give the bits of the
+    persistent kernel, and setting a schedule brings that kernel back."""
+    torch = torch_cuda
+    shapes, gap = DIRECT_PLANS[name]
+    offs, end = [], 0
+    for r, c in shapes:
+        offs.append(end)
+        end += r * c * 8 + gap
+    x = torch.from_numpy(wl.complex_uniform(1, end // 8, 7).reshape(-1)).cuda()
+    s = torch.cuda.current_stream().cuda_stream
+    got = []
+    for pin in (False, True):
+        src = x.clone()
+        dst = src if inplace else torch.zeros_like(src)
+        b = g.Batch(ctx, [src.data_ptr() + o for o in offs], [dst.data_ptr() + o for o in offs],
+                    shapes, flags)
+        if pin:
+            b.set_variant(3)
+        b.execute(s)
+        assert b.status(s) == 0
+        if not inplace:
+            assert torch.equal(src, x)
+        got.append(dst.cpu().numpy())
+        b.close()
+    assert np.array_equal(got[0].view(np.uint32), got[1].view(np.uint32))
+    if gap and not inplace:  # nothing between the images is written
+        for o, (r, c) in zip(offs, shapes):
+            assert not got[0][(o // 8 + r * c):(o // 8 + r * c + gap // 8)].any()
+
+
+def test_tuned_context_keeps_a_plan_on_the_persistent_kernel(ctx, torch_cuda):
+    """A plan's bits do not depend on the context's pass schedules."""
+    torch = torch_cuda
+    shapes = [(256, 512)] * 3
+    b, xs, _, _, plain = _run_batch(ctx, torch, shapes, (0,))
+    b.close()
+    ctx.set_fft_schedule(256, 512, 1, 1)
+    try:
+        b, _, _, _, tuned = _run_batch(ctx, torch, shapes, (0,))
+        b.close()
+    finally:
+        ctx.set_fft_schedule(256, 512, 0, 0)
+    for p, t in zip(plain, tuned):
+        assert np.array_equal(p.view(np.uint32), t.view(np.uint32))
