@@ -317,7 +317,8 @@ def schedule_available(length: int, schedule: int, along_cols: bool) -> bool:
 
 class Batch:
     """A batch plan (glsfft_batch): uneven-size images through 1-2 transforms,
-    one persistent launch, captured into a CUDA graph."""
+    one persistent launch (or, for small plans, batched pass launches),
+    captured into a CUDA graph."""
 
     def __init__(self, ctx: Context, srcs, dsts, shapes, flags=(0,)):
         n = len(srcs)
@@ -470,8 +471,8 @@ class Server:
         return out
 
     def set_frame_read(self, direct: bool) -> None:
-        """True (the default): the row kernel reads page-locked host frames
-        itself (no copy-engine transfer); False: a copy-engine transfer."""
+        """True (the default): the GPU's own kernels read page-locked host
+        frames (no copy-engine transfer); False: a copy-engine transfer."""
         check(lib().glsfft_server_set_frame_read(self.handle, int(bool(direct))),
               "server_set_frame_read")
 

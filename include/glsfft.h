@@ -563,9 +563,10 @@ GLSFFT_API int glsfft_server_replay_traced(glsfft_server server, int n, const do
 
 /*
  * How requests bring their frame to the device (no reference counterpart).
- * 1 (the default): the windowed row pass reads the frame from host memory
- * itself, for frames in page-locked memory (cudaHostAlloc /
- * cudaHostRegister; other frames are copied).  0: a copy-engine transfer
+ * 1 (the default): the GPU's own kernels read the frame from host memory --
+ * the windowed row pass or, for a large frame while other requests are in
+ * flight, a copy kernel before it -- for frames in page-locked memory
+ * (cudaHostAlloc / cudaHostRegister; other frames are copied).  0: a copy-engine transfer
  * into the request's workspace, then the row pass.  On GB300 the copy path
  * showed H2D tails of several milliseconds under load with many distinct
  * frames, the direct read did not; the copy path sustains more pairs per
