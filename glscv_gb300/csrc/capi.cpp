@@ -245,7 +245,8 @@ int glsfft::fft2d_launch(glsfft_context ctx, const void *src, void *dst, int row
         a.cols = cols;
         a.scale = scale ? 1.0f / (float)cols : 1.0f;
         a.flags = (inv ? PF_CONJ_IN : 0u) | (inv && !do_cols ? PF_CONJ_OUT : 0u) |
-                  (shift ? PF_SHIFT_COLS : 0u);
+                  (shift ? PF_SHIFT_COLS : 0u) |
+                  evict_in(src == dst ? 0 : count * src_step, count * dst_step, count);
         a.tw = ctx->d_tw;
         a.err = ctx->d_status;
         a.stall_ns = ctx->stall_ns;

@@ -44,7 +44,22 @@ enum : unsigned {
     PF_SHIFT_ROWS = 1u << 2,
     PF_SHIFT_COLS = 1u << 3,
     PF_F1_SPECTRUM = 1u << 4,
+    PF_EVICT_IN = 1u << 5,  // row passes: the input leaves the L2 first
 };
+
+// PF_EVICT_IN (2048- and 4096-point rows) where a row pass's input and result
+// overflow the 129 MB L2 and the result alone does not: the input is read
+// once, and the lines it leaves behind push out the result's rows that the
+// column pass reads next.  Measured on GB300, forward + inverse: 2048 x 4096
+// 110.1 -> 105.0 us, 4096 x 2048 128.0 -> 122.1, 40 x 64x4096 98.8 -> 91.2, one
+// 4096^2 241.0 -> 236.1.  Not where both fit, as a caller that transforms the
+// same image again would lose it (2048^2 forward 26.4 -> 27.4), nor for larger
+// results (8 x 1024x2048 197.4 -> 199.0).  1024-point rows gain less than the
+// policy operand costs 1024^2 (17.8 -> 18.0).
+inline unsigned evict_in(size_t in_bytes, size_t out_bytes, int images) {
+    constexpr size_t kL2 = size_t(1) << 27;
+    return in_bytes + out_bytes >= kL2 && (out_bytes < kL2 || images == 1) ? PF_EVICT_IN : 0u;
+}
 
 struct PassArgs {
     const void *in0;

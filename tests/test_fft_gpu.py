@@ -172,3 +172,22 @@ def test_errors_on_device(ctx, torch_cuda):
     with pytest.raises(g.GlsError) as e:
         ctx.fft2d(d.data_ptr(), d.data_ptr(), 8, 8, 8)
     assert e.value.status == 1
+
+
+@pytest.mark.parametrize("count,rows,cols", [(1, 4096, 4096), (1, 4096, 2048), (63, 64, 4096),
+                                             (64, 64, 4096), (65, 64, 4096)])
+def test_input_policy_of_large_images_changes_no_bit(ctx, torch_cuda, count, rows, cols):
+    """The row pass's input policy (sizes around where it applies) changes no
+    bit: image k of a batch equals the same image alone, in place and not."""
+    torch = torch_cuda
+    s = torch.cuda.current_stream().cuda_stream
+    x = torch.view_as_complex(torch.randn(count, rows, cols, 2, device="cuda"))
+    y = torch.empty_like(x)
+    ctx.fft2d_batched(x.data_ptr(), y.data_ptr(), count, rows, cols, 0, s)
+    one = torch.empty_like(x[0])
+    for k in {0, count - 1}:
+        ctx.fft_rows(x[k].data_ptr(), one.data_ptr(), rows, cols, 0, s)
+        ctx.fft_cols(one.data_ptr(), one.data_ptr(), rows, cols, 0, s)
+        assert torch.equal(torch.view_as_real(one), torch.view_as_real(y[k]))
+    ctx.fft2d_batched(x.data_ptr(), x.data_ptr(), count, rows, cols, 0, s)
+    assert torch.equal(torch.view_as_real(x), torch.view_as_real(y))
