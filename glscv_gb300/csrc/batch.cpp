@@ -303,6 +303,22 @@ int glsfft::make_tmap_2d(void *tmap128, const void *base, long long width, long 
     return r == CUDA_SUCCESS ? GLSFFT_SUCCESS : GLSFFT_ERROR_CUDA;
 }
 
+int glsfft::make_tmap_rows(void *tmap128, const void *base, long long width, long long height,
+                           int box_w, int box_rows) {
+    auto enc = tmap_encoder();
+    if (!enc || height % 256 || box_rows % 256) return GLSFFT_ERROR_CUDA;
+    const cuuint64_t pitch = (cuuint64_t)width * sizeof(float2);
+    cuuint64_t dims[3] = {(cuuint64_t)width, 256, (cuuint64_t)(height / 256)};
+    cuuint64_t strides[2] = {pitch, 256 * pitch};
+    cuuint32_t box[3] = {(cuuint32_t)box_w, 256, (cuuint32_t)(box_rows / 256)};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = enc(reinterpret_cast<CUtensorMap *>(tmap128), CU_TENSOR_MAP_DATA_TYPE_UINT64, 3,
+                     const_cast<void *>(base), dims, strides, box, estr,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? GLSFFT_SUCCESS : GLSFFT_ERROR_CUDA;
+}
+
 int glsfft::make_column_tmap(void *tmap128, const void *img, int rows, int cols) {
     const int w = kBatchTileElems / rows;     // columns per tile
     const int br = rows < 256 ? rows : 256;   // box height (TMA box dims <= 256)

@@ -137,6 +137,11 @@ cudaError_t launch_stream_pass(int n, bool cols, const PassArgs &a, int images, 
 // copies (batch.cpp).  GLSFFT_SUCCESS or an error status.
 int make_tmap_2d(void *tmap128, const void *base, long long width, long long height, int box_w,
                  int box_h);
+// The same with boxes higher than the 256 elements a box dimension may have:
+// a 3-D map (width, 256, height / 256) whose box is box_w x box_rows; height
+// and box_rows are multiples of 256.
+int make_tmap_rows(void *tmap128, const void *base, long long width, long long height, int box_w,
+                   int box_rows);
 
 // SMs of the current device (0 on failure), looked up once per device.
 int sm_count();

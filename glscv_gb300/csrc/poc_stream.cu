@@ -61,11 +61,8 @@ __global__ void __launch_bounds__(kPocThreads, 1)
     // both spectra of one tile: y (in1) into buffer 1, x (in0) into buffer 2
     auto issue = [&](int which) {
         mbar_arrive_tx(full, 2 * kPocTileBytes);
-#pragma unroll
-        for (int b = 0; b < N / 256; b++) {
-            tensor2d_g2s(buf1 + b * 256 * W, &maps.in1, which * W, b * 256, full);
-            tensor2d_g2s(buf2 + b * 256 * W, &maps.in0, which * W, b * 256, full);
-        }
+        tensor3d_g2s(buf1, &maps.in1, which * W, 0, 0, full);
+        tensor3d_g2s(buf2, &maps.in0, which * W, 0, 0, full);
     };
     if (tid == 0) {
         mbar_init(full, 1);
@@ -117,8 +114,7 @@ __global__ void __launch_bounds__(kPocThreads, 1)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (tid == 0) {
-#pragma unroll
-            for (int b = 0; b < N / 256; b++) tensor2d_s2g(&maps.out, tile * W, b * 256, buf0 + b * 256 * W);
+            tensor3d_s2g(&maps.out, tile * W, 0, 0, buf0);
             bulk_commit();
         }
     }
@@ -129,12 +125,12 @@ template <int N>
 cudaError_t poc_stream_t(const PassArgs &a, cudaStream_t s) {
     constexpr int W = kPocTile / N;
     PocMaps maps{};
-    if (make_tmap_2d(&maps.in0, a.in0, a.cols, a.rows, W, 256) != GLSFFT_SUCCESS ||
-        make_tmap_2d(&maps.in1, a.in1, a.cols, a.rows, W, 256) != GLSFFT_SUCCESS)
+    if (make_tmap_rows(&maps.in0, a.in0, a.cols, a.rows, W, N) != GLSFFT_SUCCESS ||
+        make_tmap_rows(&maps.in1, a.in1, a.cols, a.rows, W, N) != GLSFFT_SUCCESS)
         return cudaErrorNotSupported;
     if (a.out0 == a.in0) maps.out = maps.in0;
     else if (a.out0 == a.in1) maps.out = maps.in1;
-    else if (make_tmap_2d(&maps.out, a.out0, a.cols, a.rows, W, 256) != GLSFFT_SUCCESS)
+    else if (make_tmap_rows(&maps.out, a.out0, a.cols, a.rows, W, N) != GLSFFT_SUCCESS)
         return cudaErrorNotSupported;
     constexpr size_t smem = 128 + 3 * kPocBuf + 16;
     auto kern = poc_stream_cols<N>;

@@ -110,5 +110,13 @@ __device__ __forceinline__ void tensor2d_g2s(void *dst, const void *tmap, int x,
         "l"(tmap), "r"(x), "r"(y), "r"(smem_u32(bar))
         : "memory");
 }
+__device__ __forceinline__ void tensor3d_g2s(void *dst, const void *tmap, int x, int y, int z,
+                                             unsigned long long *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+            smem_u32(dst)),
+        "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+        : "memory");
+}
 
 }  // namespace glsfft
