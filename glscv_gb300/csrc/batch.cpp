@@ -288,8 +288,13 @@ PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
 
 }  // namespace
 
+static CUtensorMapSwizzle chunk_swizzle(bool on, int box_w) {
+    return !on ? CU_TENSOR_MAP_SWIZZLE_NONE
+               : box_w <= 4 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B;
+}
+
 int glsfft::make_tmap_2d(void *tmap128, const void *base, long long width, long long height,
-                         int box_w, int box_h) {
+                         int box_w, int box_h, bool swizzle) {
     auto enc = tmap_encoder();
     if (!enc) return GLSFFT_ERROR_CUDA;
     cuuint64_t dims[2] = {(cuuint64_t)width, (cuuint64_t)height};
@@ -298,13 +303,13 @@ int glsfft::make_tmap_2d(void *tmap128, const void *base, long long width, long 
     cuuint32_t estr[2] = {1, 1};
     CUresult r = enc(reinterpret_cast<CUtensorMap *>(tmap128), CU_TENSOR_MAP_DATA_TYPE_UINT64, 2,
                      const_cast<void *>(base), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, chunk_swizzle(swizzle, box_w),
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? GLSFFT_SUCCESS : GLSFFT_ERROR_CUDA;
 }
 
 int glsfft::make_tmap_rows(void *tmap128, const void *base, long long width, long long height,
-                           int box_w, int box_rows) {
+                           int box_w, int box_rows, bool swizzle) {
     auto enc = tmap_encoder();
     if (!enc || height % 256 || box_rows % 256) return GLSFFT_ERROR_CUDA;
     const cuuint64_t pitch = (cuuint64_t)width * sizeof(float2);
@@ -314,7 +319,7 @@ int glsfft::make_tmap_rows(void *tmap128, const void *base, long long width, lon
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = enc(reinterpret_cast<CUtensorMap *>(tmap128), CU_TENSOR_MAP_DATA_TYPE_UINT64, 3,
                      const_cast<void *>(base), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, chunk_swizzle(swizzle, box_w),
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? GLSFFT_SUCCESS : GLSFFT_ERROR_CUDA;
 }

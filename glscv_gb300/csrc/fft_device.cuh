@@ -185,6 +185,7 @@ template <> struct Dft<16> {
 // Barrier policies for the exchanges: the whole block, or only the 256
 // compute threads of a warp-specialised block (named barrier 1).
 struct SyncBlock {
+    static constexpr bool kTurns = false;
     __device__ __forceinline__ void operator()() const { __syncthreads(); }
 };
 // Lines of T consecutive threads, LINES of them per block: a line's exchange
@@ -193,6 +194,7 @@ struct SyncBlock {
 // drift apart and one's shared-memory traffic overlaps another's arithmetic.
 template <int T, int LINES>
 struct SyncLines {
+    static constexpr bool kTurns = false;
     __device__ __forceinline__ void operator()() const {
         if constexpr (T <= 32) __syncwarp();
         else if constexpr (LINES <= 15)
@@ -201,8 +203,34 @@ struct SyncLines {
     }
 };
 struct SyncCompute256 {
+    static constexpr bool kTurns = false;
     __device__ __forceinline__ void operator()() const {
         asm volatile("bar.sync 1, 256;" ::: "memory");
+    }
+};
+
+// Two groups of HALF threads (whole warps) that take turns on one exchange
+// buffer, each for its own lines: group 0's exchange after pass 0, group 1's,
+// group 0's after pass 1 and so on, so that one group's shared-memory traffic
+// runs beside the other's arithmetic.  take<p> waits before the stores of the
+// exchange after pass p, give<p> follows its loads; a block barrier stands
+// between a run's last exchange and the next use of the buffer.
+template <int HALF>
+struct SyncTurns {
+    static constexpr bool kTurns = true;
+    __device__ __forceinline__ static bool second() { return threadIdx.x >= HALF; }
+    __device__ __forceinline__ void operator()() const {
+        asm volatile("bar.sync %0, %1;" ::"r"(second() ? 2 : 1), "n"(HALF) : "memory");
+    }
+    template <int p>
+    __device__ __forceinline__ void take() const {
+        if (second()) asm volatile("bar.sync 3, %0;" ::"n"(2 * HALF) : "memory");
+        else if (p > 0) asm volatile("bar.sync 4, %0;" ::"n"(2 * HALF) : "memory");
+    }
+    template <int p, bool LAST>
+    __device__ __forceinline__ void give() const {
+        if (!second()) asm volatile("bar.arrive 3, %0;" ::"n"(2 * HALF) : "memory");
+        else if (!LAST) asm volatile("bar.arrive 4, %0;" ::"n"(2 * HALF) : "memory");
     }
 };
 
@@ -415,6 +443,10 @@ struct LineFft {
                 for (int r = 0; r < R; r++) v[r] = x[s + r * S];
                 if constexpr (Ns > 1) twiddle<p, R, Ns>(tw, j & (Ns - 1), v);
                 Dft<R>::run(v);
+                if constexpr (Sync::kTurns && !last) {
+                    static_assert(S == 1 && !Sm::kSplit, "one butterfly per thread and exchange");
+                    sync.template take<p>();
+                }
                 if constexpr (last || Sm::kSplit) {
 #pragma unroll
                     for (int r = 0; r < R; r++) x[s + r * S] = v[r];
@@ -436,7 +468,8 @@ struct LineFft {
                 for (int m = 0; m < E; m++) x[m] = in[slot_step<Sm, T>(m)];
                 // the next exchange overwrites the buffer; after the last one
                 // the caller syncs before it writes the buffer again
-                if constexpr (p + 2 < P) sync();
+                if constexpr (Sync::kTurns) sync.template give<p, (p + 2 >= P)>();
+                else if constexpr (p + 2 < P) sync();
                 pass<p + 1>(x, t, sm, tw);
             }
         }

@@ -14,9 +14,15 @@
 //     mbarrier;
 //   * every thread copies its 16 values of one column to registers, the
 //     block syncs, and thread 0 at once issues the next tile's copy;
-//   * the Stockham passes exchange through a separate float buffer, real and
-//     imaginary parts in turn (half the shared memory of a complex exchange,
-//     so stage + exchange fit one SM: 128 KB + 68 KB);
+//   * the Stockham passes exchange through a separate buffer of half the
+//     tile's size, so that stage + exchange fit one SM (128 KB + 68 KB).  For
+//     complex results the threads are two groups, each with half the columns,
+//     that take turns on it (SyncTurns); for log-magnitudes, whose register
+//     stores want a warp to have whole row segments, all columns exchange
+//     together, real and imaginary parts one after the other.  GB300, there
+//     and back, halves -> turns: 4 x 2048^2 233.5 -> 226.3 us, 4096 x 1024
+//     65.1 -> 64.2, 4096^2 231.6 -> 229.1; the 4096^2 display 135.7 -> 164.4,
+//     and 152.1 with its stores by the TMA;
 //   * complex results go out the same way: a quarter of the tile's rows at a
 //     time is laid out in one of two halves of the exchange buffer and stored
 //     by the TMA while the next quarter is written and the next tile read.
@@ -50,14 +56,22 @@ template <int N>
 __host__ __device__ constexpr int stream_lines() {
     return (int)(kStreamTileBytes / (N * sizeof(float2)));
 }
+// Complex results: the exchanges by turns; log-magnitudes: in halves (above).
+template <int ST>
+__host__ __device__ constexpr bool stream_turns() {
+    return ST == ST_C2;
+}
+// half the tile's columns at once, or all, one component at a time
 template <int N>
 __host__ __device__ constexpr size_t stream_xchg_bytes() {
-    constexpr size_t b = sizeof(float) * (size_t)col_split_floats(stream_lines<N>() * N);
+    static_assert(sizeof(float) * (size_t)col_split_floats(stream_lines<N>() * N) <=
+                  sizeof(float2) * (size_t)padded_count(stream_lines<N>() / 2 * N), "exchange buffer");
+    constexpr size_t b = sizeof(float2) * (size_t)padded_count(stream_lines<N>() / 2 * N);
     return (b + 15) & ~size_t(15);
 }
 template <int N>
 __host__ __device__ constexpr size_t stream_smem() {
-    return 128 + kStreamTileBytes + stream_xchg_bytes<N>() + 16;
+    return 512 + kStreamTileBytes + stream_xchg_bytes<N>() + 16;
 }
 template <int N, int E>
 __host__ __device__ constexpr int stream_threads() {
@@ -107,11 +121,11 @@ __global__ void __launch_bounds__(stream_threads<N, E>(), 1)
     static_assert(N % 256 == 0, "column tiles are read as 256-row boxes");
     static_assert(ST == ST_C2 || ST == ST_LOGMAG_MINMAX, "stream store modes");
     extern __shared__ unsigned char stream_raw[];
-    // 128-byte aligned stage; offsetting the shared array itself (not a cast
+    // 512-byte aligned stage (the period of the boxes' swizzle); offsetting the shared array itself (not a cast
     // integer) keeps the compiler's shared-window addressing
-    unsigned char *base = stream_raw + ((128u - (smem_u32(stream_raw) & 127u)) & 127u);
+    unsigned char *base = stream_raw + ((512u - (smem_u32(stream_raw) & 511u)) & 511u);
     float2 *stage = reinterpret_cast<float2 *>(base);
-    float *xch = reinterpret_cast<float *>(base + kStreamTileBytes);
+    float2 *xch = reinterpret_cast<float2 *>(base + kStreamTileBytes);
     unsigned long long *full =
         reinterpret_cast<unsigned long long *>(base + kStreamTileBytes + stream_xchg_bytes<N>());
 
@@ -119,7 +133,17 @@ __global__ void __launch_bounds__(stream_threads<N, E>(), 1)
     const int tid = threadIdx.x;
     const int tpi = a.cols / L;  // tiles per image
     const int total = tpi * images;
-    const int l = tid % L, t = tid / L;  // column within the tile, position thread
+    // c: column among the thread's group's, t: position thread, l: column of
+    // the tile, slot: where row t of a box has that column.  With turns, a
+    // group has every other 16-byte pair of columns, and the boxes' 16-byte
+    // chunks are permuted by the TMA (rows of 32 or 64 bytes: its 32B or 64B
+    // mode), so that a group's accesses fall on distinct banks.
+    constexpr bool TURNS = stream_turns<ST>();
+    constexpr int HALF = L / 2 * T;
+    const int c = TURNS ? tid % HALF % (L / 2) : tid % L;
+    const int t = TURNS ? tid % HALF / (L / 2) : tid / L;
+    const int l = TURNS ? 4 * (c / 2) + 2 * (tid / HALF) + c % 2 : c;
+    const int slot = t * L + (!TURNS ? l : l ^ ((L == 4 ? t >> 2 & 1 : t >> 1 & 3) << 1));
 
     if (tid == 0) {
         mbar_init(full, 1);
@@ -149,14 +173,17 @@ __global__ void __launch_bounds__(stream_threads<N, E>(), 1)
         parity ^= 1u;
         float2 x[E];
 #pragma unroll
-        for (int m = 0; m < E; m++) x[m] = stage[(t + m * T) * L + l];
+        for (int m = 0; m < E; m++) x[m] = stage[slot + m * T * L];
         if (tid == 0) bulk_wait_read<0>();  // the exchange buffer is free
         __syncthreads();  // every thread has its values: the stage is free
         const int next = tile + gridDim.x;
         if (tid == 0 && next < total) stream_issue<N, false>(maps, a, next, tpi, stage, full);
 
         conj_line(x, a.flags & PF_CONJ_IN);
-        LineFft<N, E, SyncBlock, 4>::run(x, t, ColSmF<L>{xch, l}, a.tw);
+        if constexpr (TURNS)
+            LineFft<N, E, SyncTurns<HALF>, 4>::run(x, t, ColSm<L / 2>{xch, c}, a.tw);
+        else
+            LineFft<N, E, SyncBlock, 4>::run(x, t, ColSmF<L>{reinterpret_cast<float *>(xch), l}, a.tw);
         finish_line(x, a.scale, a.flags & PF_CONJ_OUT);
 
         const int col = (tile % tpi) * L + l;
@@ -178,13 +205,13 @@ __global__ void __launch_bounds__(stream_threads<N, E>(), 1)
             constexpr int QROWS = N / 4, QM = E / 4;
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                float2 *buf = reinterpret_cast<float2 *>(xch) + (q & 1) * (QROWS * L);
+                float2 *buf = xch + (q & 1) * (QROWS * L);
                 // q = 0: the exchange's last reads are done; from q = 2 on,
                 // the store of two quarters ago has read the buffer
                 if (q >= 2 && tid == 0) bulk_wait_read<1>();
                 if (q != 1) __syncthreads();
 #pragma unroll
-                for (int m = 0; m < QM; m++) buf[(t + m * T) * L + l] = x[q * QM + m];
+                for (int m = 0; m < QM; m++) buf[slot + m * T * L] = x[q * QM + m];
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncthreads();
                 if (tid == 0) {
@@ -212,9 +239,10 @@ cudaError_t stream_launch(const PassArgs &a, int images, cudaStream_t s) {
     constexpr int L = stream_lines<N>();
     StreamMaps maps{};
     const long long height = (long long)a.rows * images;
-    if (make_tmap_rows(&maps.in, a.in0, a.cols, height, L, N) != GLSFFT_SUCCESS) return cudaErrorNotSupported;
+    if (make_tmap_rows(&maps.in, a.in0, a.cols, height, L, N, stream_turns<ST>()) != GLSFFT_SUCCESS)
+        return cudaErrorNotSupported;
     maps.out = maps.in;
-    if (ST == ST_C2 && make_tmap_2d(&maps.out, a.out0, a.cols, height, L, 256) != GLSFFT_SUCCESS)
+    if (ST == ST_C2 && make_tmap_2d(&maps.out, a.out0, a.cols, height, L, 256, true) != GLSFFT_SUCCESS)
         return cudaErrorNotSupported;
     constexpr size_t smem = stream_smem<N>();
     auto kern = fft_stream_cols<N, E, ST>;

@@ -134,14 +134,16 @@ cudaError_t launch_stream_pass(int n, bool cols, const PassArgs &a, int images, 
 
 // A 2-D tensor map over a row-major array of 8-byte elements (width x
 // height, rows `width` elements apart) with a box_w x box_h box, for TMA
-// copies (batch.cpp).  GLSFFT_SUCCESS or an error status.
+// copies (batch.cpp); `swizzle`: the 16-byte chunks of a box's rows of 32 or
+// 64 bytes permuted (the TMA's 32B or 64B mode).  GLSFFT_SUCCESS or an error
+// status.
 int make_tmap_2d(void *tmap128, const void *base, long long width, long long height, int box_w,
-                 int box_h);
+                 int box_h, bool swizzle = false);
 // The same with boxes higher than the 256 elements a box dimension may have:
 // a 3-D map (width, 256, height / 256) whose box is box_w x box_rows; height
 // and box_rows are multiples of 256.
 int make_tmap_rows(void *tmap128, const void *base, long long width, long long height, int box_w,
-                   int box_rows);
+                   int box_rows, bool swizzle = false);
 
 // SMs of the current device (0 on failure), looked up once per device.
 int sm_count();
