@@ -9,9 +9,8 @@
 // batch (image-major, then tile) and keeps the NEXT tile's copy in flight
 // while it transforms the current one:
 //   * the tile (L columns x N rows, L * N * 8 = 128 KB) lands in a
-//     shared-memory stage as N/256 2-D tensor boxes of L x 256 (Tensor Memory
-//     Accelerator, one tensor map over the whole batch), completing on an
-//     mbarrier;
+//     shared-memory stage as one tensor box (Tensor Memory Accelerator, one
+//     tensor map over the whole batch), completing on an mbarrier;
 //   * every thread copies its 16 values of one column to registers, the
 //     block syncs, and thread 0 at once issues the next tile's copy;
 //   * the Stockham passes exchange through a separate buffer of half the

@@ -27,7 +27,7 @@ static cudaError_t poc_t(const PassArgs &a, cudaStream_t s) {
 cudaError_t launch_poc_cols(int n, const PassArgs &a, cudaStream_t s) {
     // more tiles than SMs: the persistent pass, whose blocks copy the next
     // tile while they finish one.  GB300, us a synchronous call, this / the
-    // plain kernel: 2048^2 83.4 / 89.4, 2048 x 4096 151 / 170, 4096^2 315 /
+    // plain kernel: 2048^2 82.6 / 89.4, 2048 x 4096 148 / 170, 4096^2 297 /
     // 387, 2048 x 1024 48.7 / 50.0, 1024 x 2048 49.0 / 49.0; with one tile per
     // SM or fewer there is nothing to overlap: 1024^2 33.3 / 31.9.
     if ((long long)a.cols * n > 8192LL * sm_count() && poc_stream_applies(n, a)) return launch_poc_stream(n, a, s);
