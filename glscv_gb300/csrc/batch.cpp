@@ -111,27 +111,45 @@ int grid_for(int device, int variant) {
 }
 
 // Runs of equal images at a constant, non-overlapping distance in src and in
-// dst, each a batched pass launch; empty when there are more than one per
-// graph branch or when the persistent kernel is the better one.
+// dst, for batched pass launches; empty when the persistent kernel is the
+// better one.
 //
 // A pass boundary costs a launch about 1 us and the work list, with its claim,
-// dependency poll and TMA round trips, about 5 us, so the launches win until
-// the passes no longer find the images in L2: up to 64 MiB of images (128 MiB
-// with their source).  Measured on GB300, us per execution, launches against
-// the persistent kernel: 2 x 256x512 forward 9.3 / 18.7, 16 x 256^2 12.4 /
-// 18.6, 8 x 512^2 16.5 / 27.4, 8 x 1024^2 50.3 / 54.4, there and back 2 x
-// 256x512 12.4 / 30.9, 8 x 1024^2 90.2 / 91.2; beyond: 12 x 1024^2 there and
-// back 145.5 / 143.7, 96 x 64x2048 forward 68.7 / 63.7, 256 x 256^2 88.2 /
-// 78.0.  Images of the one-launch FFT gain at any size (4000 x 64^2 forward
-// 63.6 / 86.2, there and back 123 / 157).
-//
-// Runs on parallel branches: 4 x 1024^2 in separate buffers 30.8 / 37.0, 4 x
-// 256^2 13.5 / 18.5, three mixed sizes 21.3 / 26.7; with 12 mixed sizes the
-// launches themselves take as long as the persistent kernel (42.1 / 37.7).
-constexpr size_t kDirectBytes = size_t(64) << 20;
-constexpr size_t kDirectBranches = 4;
+// dependency poll and TMA round trips, about 5 us, so the launches win while
+// the passes find the images in L2.  Measured on GB300, us per execution,
+// launches against the persistent kernel:
+//   * up to 64 MiB of images (128 MiB with their sources; 48 MiB there and
+//     back), at most eight runs, each a launch per pass on a graph branch of its own: 2 x 256x512 forward
+//     8.2 / 17.7, 16 x 256^2 12.4 / 18.6, 8 x 512^2 16.5 / 27.4; 8 x 1024^2
+//     49.3 / 52.5 in one run, 45.7 in eight; eight mixed sizes 18.2 .. 33.8 /
+//     20.8 .. 35.1, there and back 30.7 .. 60.6 / 35.4 .. 62.2; with twelve the
+//     launches themselves take as long as the persistent kernel (39 / 38).
+//   * one larger run in pieces of 3 Mpx (24 MiB), each through all its passes
+//     before the next, on two branches, so that the pieces in flight stay in
+//     L2: 24 x 1024^2 120 / 133, there and back 230 / 243; 96 x 512^2
+//     114 / 124 and 216 / 233; 384 x 256^2 93 / 107 and 165 / 186; 1024 x 256^2
+//     237 / 266 and 428 / 474; 12 x 1024x2048 132 / 143 and 250 / 270.  As one
+//     launch per pass 24 x 1024^2 took 142 and 280; pieces of 2 or 4 Mpx or
+//     more branches are up to 10 % slower.
+//     Not 1024-row images with a column-tiled workspace beyond 24 Mpx (64 x
+//     1024^2 there and back 602 / 608, 512 x 1024x128 592 / 578) or of fewer
+//     than 256 columns (384 x 1024x64 265 / 260, 56 x 1024x128 75 / 73).  Over
+//     338 runs of 15 sizes, 0.4 .. 50 Mpx, the default came out 1.20 times as
+//     fast as the persistent kernel; the slowest beside that 1024x128, which
+//     this line then left out, 50 x 512x2048 480 / 472.
+//   * images of the one-launch FFT gain at any total (4000 x 64^2 forward 63.6
+//     / 86.2, there and back 123 / 157);
+//   * images of 32 columns up to 16 MiB, of 16 up to 4, whose rows the pass
+//     kernels read in short pieces: 64 x 512x32 there and back 1.25 times as
+//     fast, 256 x 512x32 1.05, 505 x 512x32 0.96; 64 x 512x16 1.56, 128 x
+//     512x16 0.94.
+constexpr size_t direct_bytes(size_t transforms) { return size_t(transforms > 1 ? 48 : 64) << 20; }
+constexpr size_t kNarrowBytes = size_t(4) << 20;
+constexpr size_t kDirectBranches = 8;
+constexpr size_t kPiecePixels = size_t(3) << 20;
 
-std::vector<glsfft_batch_s::Segment> direct_segments(const std::vector<BatchImage> &images) {
+std::vector<glsfft_batch_s::Segment> direct_segments(const std::vector<BatchImage> &images,
+                                                     size_t transforms) {
     std::vector<glsfft_batch_s::Segment> segs;
     std::map<std::pair<int, int>, size_t> last;  // the size's run that may still grow
     size_t bytes = 0;
@@ -161,8 +179,28 @@ std::vector<glsfft_batch_s::Segment> direct_segments(const std::vector<BatchImag
         last[{im.rows, im.cols}] = segs.size();
         segs.push_back({im.src, im.dst, im.rows, im.cols, 1, 0, 0});
     }
-    if (bytes > kDirectBytes && !fused) segs.clear();
-    return segs;
+    if (fused || segs.empty()) return segs;
+    for (const auto &sg : segs)
+        if (sg.cols < 64 && bytes > kNarrowBytes * (sg.cols / 16) * (sg.cols / 16)) return {};
+    if (bytes <= direct_bytes(transforms)) return segs;
+    const auto &sg = segs[0];
+    const bool tiled = batch_tiled_ok(sg.rows, sg.cols);
+    if (segs.size() > 1 || (tiled && (sg.cols < 256 || bytes > 8 * (size_t(24) << 20)))) return {};
+    // an even number of pieces, as equal as they come, for the two branches
+    const int pairs = (int)((bytes / 8 + 2 * kPiecePixels - 1) / (2 * kPiecePixels));
+    if (pairs > 256) return {};  // a graph of thousands of launches
+    const int n = std::min(sg.count, 2 * pairs);
+    std::vector<glsfft_batch_s::Segment> pieces;
+    for (int k = 0; k < n; k++) {
+        const int first = (int)((long long)sg.count * k / n),
+                  end = (int)((long long)sg.count * (k + 1) / n);
+        glsfft_batch_s::Segment p = sg;
+        p.src = static_cast<const char *>(sg.src) + first * sg.src_step;
+        p.dst = static_cast<char *>(sg.dst) + first * sg.dst_step;
+        p.count = end - first;
+        pieces.push_back(p);
+    }
+    return pieces;
 }
 
 // The launches stand in for the persistent kernel only with the context's
@@ -177,45 +215,41 @@ bool use_direct(glsfft_batch plan) {
     return true;
 }
 
-// The runs' pass launches, one branch of the graph each.
+// The runs' launches on a branch of the graph each, the pieces' on two.
 int record_direct(glsfft_batch plan, cudaStream_t s) {
-    const size_t extra = plan->segments.size() - 1;
-    cudaStream_t br[kDirectBranches] = {};
-    cudaEvent_t ev[kDirectBranches] = {};
-    cudaEvent_t fork = nullptr;
+    const auto &segs = plan->segments;
+    size_t bytes = 0;
+    for (const auto &sg : segs) bytes += sizeof(float2) * (size_t)sg.rows * sg.cols * sg.count;
+    const size_t n = std::min(segs.size(), bytes > direct_bytes(plan->flags.size()) ? 2 : kDirectBranches);
+    cudaStream_t br[kDirectBranches] = {s};
+    cudaEvent_t ev[kDirectBranches] = {};  // ev[0]: the fork
     cudaError_t e = cudaSuccess;
-    if (extra) {
-        e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaEventRecord(fork, s);
+    for (size_t i = 0; i < n && n > 1 && e == cudaSuccess; i++) {
+        e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
+        if (e == cudaSuccess && i) e = cudaStreamCreateWithFlags(&br[i], cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = i ? cudaStreamWaitEvent(br[i], ev[0], 0) : cudaEventRecord(ev[0], s);
     }
-    int st = GLSFFT_SUCCESS;
-    for (size_t i = 0; i <= extra && e == cudaSuccess && !st; i++) {
-        const auto &sg = plan->segments[i];
-        if (i) {
-            e = cudaStreamCreateWithFlags(&br[i], cudaStreamNonBlocking);
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(br[i], fork, 0);
-            if (e != cudaSuccess) break;
-        }
-        cudaStream_t b = i ? br[i] : s;
+    int st = cuda_status(e);
+    for (size_t k = 0; k < segs.size() && !st; k++) {
+        const auto &sg = segs[k];
         const void *src = sg.src;
         size_t step = sg.src_step;
-        for (int f : plan->flags) {
-            st = fft2d_launch(plan->ctx, src, sg.dst, sg.rows, sg.cols, f, false, b, sg.count, step,
-                              sg.dst_step);
-            if (st) break;
+        for (size_t t = 0; t < plan->flags.size() && !st; t++) {
+            st = fft2d_launch(plan->ctx, src, sg.dst, sg.rows, sg.cols, plan->flags[t], false,
+                              br[k % n], sg.count, step, sg.dst_step);
             src = sg.dst;
             step = sg.dst_step;
         }
-        if (i && !st) e = cudaEventRecord(ev[i], b);
     }
-    for (size_t i = 1; i <= extra && e == cudaSuccess && !st; i++) e = cudaStreamWaitEvent(s, ev[i], 0);
-    if (!st) st = cuda_status(e);
-    for (size_t i = 1; i <= extra; i++) {
+    for (size_t i = 1; i < n && !st; i++) {
+        e = cudaEventRecord(ev[i], br[i]);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ev[i], 0);
+        st = cuda_status(e);
+    }
+    for (size_t i = 0; i < n; i++) {
         if (ev[i]) cudaEventDestroy(ev[i]);
-        if (br[i]) cudaStreamDestroy(br[i]);
+        if (i && br[i]) cudaStreamDestroy(br[i]);
     }
-    if (fork) cudaEventDestroy(fork);
     return st;
 }
 
@@ -494,7 +528,7 @@ int glsfft_batch_create(glsfft_context ctx, int count, const void *const *srcs,
             a.claim_ahead = 0;
         }
     }
-    if (!st && plan->others.empty()) plan->segments = direct_segments(plan->images);
+    if (!st && plan->others.empty()) plan->segments = direct_segments(plan->images, plan->flags.size());
     if (!st) st = capture(plan);
     if (st) {
         if (plan->exec) cudaGraphExecDestroy(plan->exec);

@@ -322,10 +322,10 @@ typedef struct glsfft_batch_s *glsfft_batch;
  * 16 <= rows <= 1024 and 16 <= cols <= 4096 are processed by one persistent
  * launch that pulls (image, pass, tile) items from a work list, each pass of
  * an image waiting (bounded) for that image's previous pass; other shapes get
- * their own pass launches.  A plan of at most four runs of equal, evenly
- * spaced images, all of those shapes and 64 MiB together, uses batched pass
- * launches in place of the persistent one (same results) until a schedule is
- * set.  Everything is captured once into a CUDA graph.
+ * their own pass launches.  A plan of a few runs of equal, evenly spaced
+ * images, all of those shapes and 64 MiB together, or of one larger run, uses
+ * batched pass launches in place of the persistent one where that is faster
+ * (same results), until a schedule is set.  Everything is captured once into a CUDA graph.
  * No reference counterpart (glsCV transforms one texture per call).  The
  * plan keeps the pointers: the buffers must outlive it.
  */

@@ -224,6 +224,12 @@ DIRECT_PLANS = {
     "equal images with gaps": ([(16, 16)] * 9, 48),
     "four runs, interleaved": ([(64, 64), (32, 2048), (1024, 64), (512, 512)] * 2, 16),
     "two uneven sizes": ([(1024, 16), (1024, 16), (16, 4096)], 0),
+    "nine sizes": ([(64, 64), (32, 32), (16, 64), (64, 16), (128, 32), (16, 16), (16, 32),
+                    (32, 16), (32, 64)], 0),
+    "narrow images, few and many": ([(512, 32)] * 64 + [(512, 32)] * 100, 0),
+    "very narrow images": ([(1024, 16)] * 40, 0),
+    "a run in pieces, with gaps": ([(256, 1024)] * 41, 16),
+    "a run in pieces of a tiled shape": ([(1024, 256)] * 37, 0),
     "one run of the largest total": ([(512, 1024)] * 16, 0),
     "just above it": ([(512, 1024)] * 17, 0),
     "five sizes": ([(64, 64), (32, 32), (16, 64), (64, 16), (128, 32)], 0),
