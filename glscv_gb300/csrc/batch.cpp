@@ -124,7 +124,9 @@ int grid_for(int device, int variant) {
 //     49.3 / 52.5 in one run, 45.7 in eight; eight mixed sizes 18.2 .. 33.8 /
 //     20.8 .. 35.1, there and back 30.7 .. 60.6 / 35.4 .. 62.2; with twelve the
 //     launches themselves take as long as the persistent kernel (39 / 38).
-//   * one larger run in pieces of 3 Mpx (24 MiB), each through all its passes
+//   * one larger run in pieces of about 3 Mpx (24 MiB; at most 3.5, an even
+//     number of them: 14 Mpx there and back 2 .. 7 % faster in four pieces than
+//     in six, 7 Mpx 10 .. 15 % in two than in four), each through all its passes
 //     before the next, on two branches, so that the pieces in flight stay in
 //     L2: 24 x 1024^2 120 / 133, there and back 230 / 243; 96 x 512^2
 //     114 / 124 and 216 / 233; 384 x 256^2 93 / 107 and 165 / 186; 1024 x 256^2
@@ -133,10 +135,10 @@ int grid_for(int device, int variant) {
 //     more branches are up to 10 % slower.
 //     Not 1024-row images with a column-tiled workspace beyond 24 Mpx (64 x
 //     1024^2 there and back 602 / 608, 512 x 1024x128 592 / 578) or of fewer
-//     than 256 columns (384 x 1024x64 265 / 260, 56 x 1024x128 75 / 73).  Over
-//     338 runs of 15 sizes, 0.4 .. 50 Mpx, the default came out 1.20 times as
-//     fast as the persistent kernel; the slowest beside that 1024x128, which
-//     this line then left out, 50 x 512x2048 480 / 472.
+//     than 256 columns (384 x 1024x64 265 / 260, 56 x 1024x128 75 / 73), nor
+//     shorter images of 2048 columns beyond 24 Mpx (50 x 512x2048 480 / 472).
+//     Over 338 runs of 15 sizes, 0.4 .. 50 Mpx, the launches came out 1.20
+//     times as fast as the persistent kernel.
 //   * images of the one-launch FFT gain at any total (4000 x 64^2 forward 63.6
 //     / 86.2, there and back 123 / 157);
 //   * images of 32 columns up to 16 MiB, of 16 up to 4, whose rows the pass
@@ -146,7 +148,7 @@ int grid_for(int device, int variant) {
 constexpr size_t direct_bytes(size_t transforms) { return size_t(transforms > 1 ? 48 : 64) << 20; }
 constexpr size_t kNarrowBytes = size_t(4) << 20;
 constexpr size_t kDirectBranches = 8;
-constexpr size_t kPiecePixels = size_t(3) << 20;
+constexpr size_t kPiecePixels = size_t(7) << 19;
 
 std::vector<glsfft_batch_s::Segment> direct_segments(const std::vector<BatchImage> &images,
                                                      size_t transforms) {
@@ -185,7 +187,10 @@ std::vector<glsfft_batch_s::Segment> direct_segments(const std::vector<BatchImag
     if (bytes <= direct_bytes(transforms)) return segs;
     const auto &sg = segs[0];
     const bool tiled = batch_tiled_ok(sg.rows, sg.cols);
-    if (segs.size() > 1 || (tiled && (sg.cols < 256 || bytes > 8 * (size_t(24) << 20)))) return {};
+    const bool large = bytes > 8 * (size_t(24) << 20);
+    if (segs.size() > 1 || (tiled && (sg.cols < 256 || large)) ||
+        (sg.cols == 2048 && sg.rows < 1024 && large))
+        return {};
     // an even number of pieces, as equal as they come, for the two branches
     const int pairs = (int)((bytes / 8 + 2 * kPiecePixels - 1) / (2 * kPiecePixels));
     if (pairs > 256) return {};  // a graph of thousands of launches
