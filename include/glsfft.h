@@ -394,7 +394,8 @@ GLSFFT_API int glsfft_batch_workspace(glsfft_batch plan, int *tiled_images, size
  */
 GLSFFT_API int glsfft_batch_inject_stall(glsfft_batch plan, long long wait_limit_ns);
 
-/* The plan's current schedule: {variant, claim_chunk, claim_ahead, lag_items}. */
+/* The persistent kernel's current schedule: {variant, claim_chunk, claim_ahead,
+ * lag_items}, also while the plan uses pass launches in its place. */
 GLSFFT_API int glsfft_batch_get_schedule(glsfft_batch plan, int *schedule4);
 
 /*
