@@ -110,8 +110,7 @@ __device__ __forceinline__ void keys_add(float v, size_t i, unsigned long long &
     kmax = k1 > kmax ? k1 : kmax;
 }
 template <bool LOG, bool KEYS>
-__global__ void __launch_bounds__(kThreads) spec_mag_kernel(const float2 *__restrict__ a,
-                                                           float *__restrict__ d, size_t n,
+__global__ void __launch_bounds__(kThreads) spec_mag_kernel(const float2 *a, float *d, size_t n,
                                                            float offset,
                                                            unsigned long long *keys) {
     __shared__ unsigned long long red[2 * (kThreads / 32)];
@@ -204,7 +203,7 @@ int minmax_grid(size_t n);
 // a reader that reduces them itself (normalize_kernel): no reset and no
 // atomics.  The input may come from the grid before, so the wait comes first.
 template <bool PARTIAL>
-__global__ void __launch_bounds__(kThreads) minmax_kernel(const float *__restrict__ x, size_t n,
+__global__ void __launch_bounds__(kThreads) minmax_kernel(const float *x, size_t n,
                                                           unsigned long long *keys) {
     __shared__ unsigned long long red[2 * (kThreads / 32)];
     MinMaxRun run;

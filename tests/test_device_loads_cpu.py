@@ -4,7 +4,8 @@ A pass kernel launched with the programmatic-serialisation attribute starts
 while its predecessor still writes the images that it is about to read; only
 `griddepcontrol.wait` stands between.  A load may be moved above that wait when
 the source lets the compiler take it for a pure function: inline assembly
-without `volatile` and a "memory" clobber.  Whether one build's scheduling does
+without `volatile` and a "memory" clobber, or a load declared read-only for the
+kernel's lifetime (`__ldg`, `const __restrict__`).  Whether one build's scheduling does
 so shows in no test result, so the sources are checked."""
 from __future__ import annotations
 
@@ -43,3 +44,13 @@ def test_asm_memory_accesses_are_ordered(path):
     for volatile, text in _asm_statements(_code(path)):
         if access.search(text):
             assert volatile and '"memory"' in text, text.strip()
+
+
+@pytest.mark.parametrize("path", [p for p in DEVICE_SOURCES if re.search(
+    r"pdl_enter\(\)|griddepcontrol\.wait", _code(p)) or p.name == "fft_kernels.cuh"], ids=lambda p: p.name)
+def test_images_are_not_declared_read_only(path):
+    """In the kernels with a dependency wait only the constant tables (uploaded
+    when the context is created) are read through the read-only path."""
+    code = _code(path)
+    for m in re.finditer(r"__ldg\(\s*(\w+)|__restrict__\s+(\w+)", code):
+        assert (m.group(1) or m.group(2)) in ("g_dft", "g_tw"), m.group(0)
