@@ -279,14 +279,16 @@ int glsfft::fft2d_launch(glsfft_context ctx, const void *src, void *dst, int row
 }
 
 // phaseCorrelate launch sequence on caller-provided scratch:
-// f1, f2: rows*cols complex each; surface: rows*cols floats; key: 8 bytes.
+// f1, f2: rows*cols complex each; surface: rows*cols floats; key: 24 bytes
+// (PassArgs::key).  err, stall_ns: the context's status word (or none) and its
+// fault injection.
 int glsfft::poc_launch(const float2 *tw, const float *src1, const float *src2,
                        const float *window, int rows, int cols, int box, float2 *f1, float2 *f2,
                        float *surface, unsigned long long *key, double *d_result,
-                       cudaStream_t s, unsigned long long *done_flag, int *err) {
-    // three launches: rows of both images; fused POC columns (which also
-    // zero the argmax key and block counter); inverse rows with the argmax
-    // and, in the last block, the centroid.  All three use programmatic
+                       cudaStream_t s, unsigned long long *done_flag, int *err,
+                       long long stall_ns) {
+    // three launches: rows of both images (which also zero the key words);
+    // fused POC columns; inverse rows with the argmax and, in the last block, the centroid.  All three use programmatic
     // dependent launch, so each grid is resident and waiting when its
     // predecessor (the previous call's last pass, for the first) ends.
     PassArgs a{};
@@ -298,6 +300,7 @@ int glsfft::poc_launch(const float2 *tw, const float *src1, const float *src2,
     a.rows = rows;
     a.cols = cols;
     a.scale = 1.0f;
+    a.key = key;
     a.tw = tw;
     a.pdl = a.spread = 1;
     cudaError_t e = launch_rows(cols, window ? LD_R1W : LD_R1, ST_C2, a, 2, s);
@@ -313,6 +316,7 @@ int glsfft::poc_launch(const float2 *tw, const float *src1, const float *src2,
     b.key = key;
     b.tw = tw;
     b.err = err;
+    b.stall_ns = stall_ns;
     b.pdl = b.spread = 1;
     e = launch_poc_cols(rows, b, s);
     if (e != cudaSuccess) return cuda_status(e);
@@ -599,7 +603,7 @@ int glsfft_phase_correlate_async(glsfft_context ctx, const float *src1, const fl
     ctx->surface = surface;
     ctx->surface_count = n;
     return poc_launch(ctx->d_tw, src1, src2, window, rows, cols, box, f1, f2, surface, key,
-                      d_result, (cudaStream_t)stream, nullptr, ctx->d_status);
+                      d_result, (cudaStream_t)stream, nullptr, ctx->d_status, ctx->stall_ns);
 }
 
 // The synchronous call's three launches into the context's mapped result.  A
@@ -630,13 +634,14 @@ static int poc_sync_launch(glsfft_context ctx, const float *src1, const float *s
     auto &pg = ctx->poc_graph;
     auto same = [&] {
         return pg.src1 == src1 && pg.src2 == src2 && pg.window == window &&
-               pg.rows == rows && pg.cols == cols && pg.box == box && pg.ws == ctx->ws;
+               pg.rows == rows && pg.cols == cols && pg.box == box && pg.ws == ctx->ws &&
+               pg.stall_ns == ctx->stall_ns;
     };
     if (!same()) {
         if (pg.exec) cudaGraphExecDestroy(pg.exec);
-        pg = {src1, src2, window, rows, cols, box, ctx->ws, nullptr, 0};
+        pg = {src1, src2, window, rows, cols, box, ctx->ws, ctx->stall_ns, nullptr, 0};
         return poc_launch(ctx->d_tw, src1, src2, window, rows, cols, box, f1, f2, surface, key,
-                          ctx->h_result_dev, s, flag, ctx->d_status);
+                          ctx->h_result_dev, s, flag, ctx->d_status, ctx->stall_ns);
     }
     if (!pg.exec && pg.repeats < kPocGraphAfter && ++pg.repeats == kPocGraphAfter) {
         if (!ctx->capture_stream &&
@@ -647,7 +652,8 @@ static int poc_sync_launch(glsfft_context ctx, const float *src1, const float *s
                 cudaSuccess) {
             cudaGraph_t graph = nullptr;
             st = poc_launch(ctx->d_tw, src1, src2, window, rows, cols, box, f1, f2, surface, key,
-                            ctx->h_result_dev, ctx->capture_stream, flag, ctx->d_status);
+                            ctx->h_result_dev, ctx->capture_stream, flag, ctx->d_status,
+                            ctx->stall_ns);
             const cudaError_t e = cudaStreamEndCapture(ctx->capture_stream, &graph);
             if (st || e != cudaSuccess || !graph ||
                 cudaGraphInstantiate(&pg.exec, graph, 0) != cudaSuccess)
@@ -658,7 +664,7 @@ static int poc_sync_launch(glsfft_context ctx, const float *src1, const float *s
     }
     if (pg.exec) return cuda_status(cudaGraphLaunch(pg.exec, s));
     return poc_launch(ctx->d_tw, src1, src2, window, rows, cols, box, f1, f2, surface, key,
-                      ctx->h_result_dev, s, flag, ctx->d_status);
+                      ctx->h_result_dev, s, flag, ctx->d_status, ctx->stall_ns);
 }
 
 int glsfft_phase_correlate(glsfft_context ctx, const float *src1, const float *src2,
@@ -697,6 +703,11 @@ int glsfft_phase_correlate(glsfft_context ctx, const float *src1, const float *s
     } else {
         cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
         if (e != cudaSuccess) return cuda_status(e);
+    }
+    if (ctx->h_result[3] < 0.0) {  // the peak index of an expired tile wait
+        ctx->surface = nullptr;
+        ctx->surface_count = 0;
+        return GLSFFT_ERROR_TIMEOUT;
     }
     *dx = ctx->h_result[0];
     *dy = ctx->h_result[1];

@@ -43,6 +43,7 @@ struct glsfft_context_s {
         const float *src1 = nullptr, *src2 = nullptr, *window = nullptr;
         int rows = 0, cols = 0, box = 0;
         const void *ws = nullptr;
+        long long stall_ns = 0;
         cudaGraphExec_t exec = nullptr;
         int repeats = 0;  // calls in a row that repeated them
     } poc_graph;
@@ -81,7 +82,8 @@ constexpr int kMaxBatch = 65535;  // grid y extent
 int poc_launch(const float2 *tw, const float *src1, const float *src2, const float *window,
                int rows, int cols, int box, float2 *f1, float2 *f2, float *surface,
                unsigned long long *key, double *d_result, cudaStream_t s,
-               unsigned long long *done_flag = nullptr, int *err = nullptr);
+               unsigned long long *done_flag = nullptr, int *err = nullptr,
+               long long stall_ns = 0);
 
 void host_pipe_destroy(HostPipe *p);  // waits for its streams, frees everything
 

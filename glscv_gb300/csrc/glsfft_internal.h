@@ -76,8 +76,10 @@ struct PassArgs {
     size_t out_img_bytes;
     float param;       // ST_LOGMAG_MINMAX: the log-magnitude offset
     // ST_RE_ARGMAX with `result` set: the last block to finish computes the
-    // phaseCorrelate centroid (box edge `box`) into result[0..4]; key[1] is
-    // the block counter (zeroed, with key[0], by the POC column pass)
+    // phaseCorrelate centroid (box edge `box`) into result[0..4].  key[0] is
+    // the argmax key, key[1] the block counter, key[2] nonzero if a tile wait
+    // of the column pass ran out (the result then says so: poc_result); the
+    // call's first row pass zeroes all three
     double *result;
     int box;
     // with `result`: set to 1 (after a system-scope fence) once result[0..4]
@@ -86,7 +88,7 @@ struct PassArgs {
     // device status word for bounded waits (the streamed passes record
     // GLSFFT_ERROR_TIMEOUT there), or null
     int *err;
-    // fault injection for tests (streamed passes): when > 0, each block
+    // fault injection for tests (the TMA-fed passes): when > 0, each block
     // leaves its first tile's copy unissued and waits this many nanoseconds
     // for it, so the wait runs out
     long long stall_ns;
@@ -119,7 +121,7 @@ cudaError_t launch_frame_copy(const float *host, float *dst, size_t n, cudaStrea
 
 // The persistent phaseCorrelate column pass (poc_stream.cu): whether it takes
 // these arguments (1024-, 2048- or 4096-point columns, whole tiles, 16-byte
-// aligned, a status word), and its launch.
+// aligned, the call's key words), and its launch.
 bool poc_stream_applies(int n, const PassArgs &a);
 cudaError_t launch_poc_stream(int n, const PassArgs &a, cudaStream_t s);
 

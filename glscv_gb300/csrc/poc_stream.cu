@@ -20,9 +20,11 @@
 // Same lines, same order of operations: the bits are the plain kernel's.
 // Measured on GB300 (a synchronous call): see launch_poc_cols.
 //
-// Every wait for a tile is bounded: on expiry the kernel records
-// GLSFFT_ERROR_TIMEOUT in the status word, waits (bounded) for its copies in
-// flight and returns.
+// Every wait for a tile is bounded: on expiry the kernel marks the call's key
+// words, from which the last pass makes a result that says so, records
+// GLSFFT_ERROR_TIMEOUT in the status word if there is one, waits (bounded) for
+// its copies in flight and returns.  Host-side fault injection (stall_ns): each
+// block's first tile is not copied, and the wait for it runs out after that.
 #include <cuda.h>
 
 #include "fft_config.h"
@@ -73,19 +75,17 @@ __global__ void __launch_bounds__(kPocThreads, 1)
     }
     __syncthreads();
     pdl_enter();
-    // the argmax key and the block counter of the inverse row pass that follows
-    if (a.key && blockIdx.x == 0 && tid == 0) {
-        a.key[0] = 0ull;
-        a.key[1] = 0ull;
-    }
-    if (tid == 0 && tile < total) issue(tile);
+    const bool inject = a.stall_ns > 0;
+    const long long limit = inject ? a.stall_ns : kPocWaitNs;
+    if (tid == 0 && tile < total && !inject) issue(tile);
     unsigned parity = 0;
     for (; tile < total; tile += gridDim.x) {
-        const bool ok = mbar_wait(full, parity, kPocWaitNs);
+        const bool ok = mbar_wait(full, parity, limit);
         if (__syncthreads_or(!ok)) {
             if (tid == 0) {
-                atomicExch(a.err, (int)GLSFFT_ERROR_TIMEOUT);
-                mbar_wait(full, parity, kPocWaitNs);
+                atomicExch(a.key + 2, 1ull);
+                if (a.err) atomicExch(a.err, (int)GLSFFT_ERROR_TIMEOUT);
+                if (!inject) mbar_wait(full, parity, kPocWaitNs);
                 bulk_wait<0>();
             }
             __syncthreads();
@@ -148,7 +148,7 @@ cudaError_t poc_stream_t(const PassArgs &a, cudaStream_t s) {
 }  // namespace
 
 bool poc_stream_applies(int n, const PassArgs &a) {
-    if ((n != 1024 && n != 2048 && n != 4096) || a.rows != n || !a.err) return false;
+    if ((n != 1024 && n != 2048 && n != 4096) || a.rows != n || !a.key) return false;
     const int w = kPocTile / n;
     auto al16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     return a.cols >= w && a.cols % w == 0 && al16(a.in0) && al16(a.in1) && al16(a.out0);

@@ -135,13 +135,13 @@ int launch_request(glsfft_server srv, const Reference &ref, const Request &rq, S
     float2 *f2 = reinterpret_cast<float2 *>(ws + Arena::round_up(4 * n));
     float *surface = reinterpret_cast<float *>(ws + Arena::round_up(4 * n) + Arena::round_up(8 * n));
     char *tail = ws + Arena::round_up(4 * n) + Arena::round_up(8 * n) + Arena::round_up(4 * n);
-    auto *key = reinterpret_cast<unsigned long long *>(tail);  // argmax key, block counter
+    auto *key = reinterpret_cast<unsigned long long *>(tail);  // PassArgs::key
     const float2 *spec = reinterpret_cast<const float2 *>(srv->d_base + ref.spec_off);
     const float *win = ref.has_window ? reinterpret_cast<const float *>(srv->d_base + ref.win_off) : nullptr;
     cudaStream_t s = slot.stream;
 
-    // the frame's way to the device, three launches (the POC column pass
-    // zeroes the argmax key; the last block of the inverse row pass computes
+    // the frame's way to the device, three launches (the row pass zeroes the
+    // key words; the last block of the inverse row pass computes
     // the centroid and writes it into the slot's mapped pinned buffer), the event
     cudaError_t e = cudaEventRecord(slot.start, s);
     if (e == cudaSuccess && rq.linked) {
@@ -166,6 +166,7 @@ int launch_request(glsfft_server srv, const Reference &ref, const Request &rq, S
     a.rows = rows;
     a.cols = cols;
     a.scale = 1.0f;
+    a.key = key;
     a.tw = srv->ctx->d_tw;
     e = launch_rows(cols, win ? LD_R1W : LD_R1, ST_C2, a, 1, s);
     if (e != cudaSuccess) return cuda_status(e);
@@ -178,7 +179,7 @@ int launch_request(glsfft_server srv, const Reference &ref, const Request &rq, S
     b.scale = 1.0f;
     b.flags = PF_F1_SPECTRUM;
     b.key = key;
-    b.err = srv->ctx->d_status;
+    b.stall_ns = srv->ctx->stall_ns;
     b.tw = srv->ctx->d_tw;
     b.pdl = 1;  // resident while the row pass drains
     e = launch_poc_cols(rows, b, s);
@@ -305,8 +306,14 @@ void poller_main(glsfft_server srv) {
                 float ms = 0.f;
                 if (cudaEventElapsedTime(&ms, slot.start, slot.done) == cudaSuccess) rq.gpu_s = 1e-3 * ms;
                 if (cudaEventElapsedTime(&ms, slot.start, slot.copied) == cudaSuccess) rq.copy_s = 1e-3 * ms;
-                rq.state = REQ_DONE;
-                srv->completed++;
+                if (rq.result[3] < 0.0) {  // a tile wait of its column pass ran out
+                    rq.state = REQ_FAILED;
+                    rq.status = GLSFFT_ERROR_TIMEOUT;
+                    srv->failed++;
+                } else {
+                    rq.state = REQ_DONE;
+                    srv->completed++;
+                }
             } else {
                 cudaGetLastError();
                 rq.state = REQ_FAILED;

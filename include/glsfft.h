@@ -80,17 +80,19 @@ GLSFFT_API int glsfft_context_set_budget(glsfft_context ctx, size_t bytes);
 GLSFFT_API int glsfft_context_workspace(glsfft_context ctx, size_t *bytes);
 
 /* Sticky status of the context's device-side bounded waits outside batch
- * plans and servers (the streamed passes' tile waits): GLSFFT_SUCCESS, or
+ * plans and servers (the tile waits of the streamed passes and of
+ * phaseCorrelate's persistent column pass): GLSFFT_SUCCESS, or
  * GLSFFT_ERROR_TIMEOUT once a wait expired (that pass's output is then
  * incomplete).  Synchronises with the device; `clear` resets the word.  No
  * reference counterpart. */
 GLSFFT_API int glsfft_device_status(glsfft_context ctx, int clear);
 
 /* Host-side fault injection for tests: with wait_limit_ns > 0, every
- * streamed pass launched on this context leaves each block's first tile copy
- * unissued and bounds the wait for it by wait_limit_ns, so the wait runs
- * out: the pass records GLSFFT_ERROR_TIMEOUT (glsfft_device_status) and
- * returns with no copy in flight; the context stays usable.  0 turns the
+ * streamed pass and persistent phaseCorrelate column pass launched on this
+ * context or its servers leaves each block's first tile copy unissued and bounds the wait for it by wait_limit_ns, so the wait runs
+ * out: the pass records GLSFFT_ERROR_TIMEOUT (glsfft_device_status; a server's
+ * request fails with it instead) and returns with no copy in flight; the
+ * context stays usable.  0 turns the
  * injection off. */
 GLSFFT_API int glsfft_context_inject_stall(glsfft_context ctx, long long wait_limit_ns);
 
@@ -461,7 +463,8 @@ GLSFFT_API int glsfft_batch_destroy(glsfft_batch plan);
  * src2, window, shape, box and workspace (the buffers' contents may change)
  * come to replay the three launches as one CUDA graph; any other call launches
  * them directly.  Not to be called from inside a stream
- * capture.
+ * capture.  GLSFFT_ERROR_TIMEOUT, with the outputs untouched, when a
+ * device-side wait of the call ran out.
  */
 GLSFFT_API int glsfft_phase_correlate(glsfft_context ctx, const float *src1, const float *src2,
                                       const float *window, int rows, int cols, int box,
@@ -470,7 +473,8 @@ GLSFFT_API int glsfft_phase_correlate(glsfft_context ctx, const float *src1, con
 /*
  * Asynchronous form: writes 5 doubles to device memory `d_result`
  * {dx, dy, response, peak row-major index, peak value}; nothing is copied
- * to the host and nothing synchronises.
+ * to the host and nothing synchronises.  When a device-side wait of the call
+ * ran out the index is -1 and the others are NaN.
  */
 GLSFFT_API int glsfft_phase_correlate_async(glsfft_context ctx, const float *src1,
                                             const float *src2, const float *window, int rows,
@@ -530,7 +534,9 @@ GLSFFT_API int glsfft_server_submit(glsfft_server server, int ref_id, const floa
 /*
  * Wait (at most timeout_s) for a request; fills {dx, dy, response, peak
  * index, peak value} and the latency from arrival to completion, then forgets
- * the ticket.  GLSFFT_ERROR_TIMEOUT when it is still running.
+ * the ticket.  GLSFFT_ERROR_TIMEOUT when it is still running; also, with the
+ * peak index -1 and the ticket forgotten, when a device-side wait of the
+ * request ran out.
  */
 GLSFFT_API int glsfft_server_wait(glsfft_server server, long long ticket, double *result5,
                                   double *latency_s, double timeout_s);
