@@ -92,7 +92,8 @@ struct PassArgs {
     // leaves its first tile's copy unissued and waits this many nanoseconds
     // for it, so the wait runs out
     long long stall_ns;
-    // a small grid is spread evenly over the SMs (launch_pass)
+    // a small grid may take other block shapes, to spread evenly over the SMs
+    // (row_lines, cols_t): not a launch beside other streams' (the server's)
     int spread;
     // launch with programmatic dependent launch (every pass kernel begins
     // with griddepcontrol.wait): the grid may become resident before its

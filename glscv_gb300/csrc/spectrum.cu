@@ -71,7 +71,7 @@ __device__ __forceinline__ float2 spec_binary_op(float2 x, float2 y) {
 template <int OP>
 __global__ void __launch_bounds__(kThreads) spec_binary_kernel(const float2 *a, const float2 *b,
                                                               float2 *d, size_t n) {
-    pdl_enter();
+    pdl_wait();
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     size_t done = 0;
@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(kThreads) spec_binary_kernel(const float2 *a, 
         if (i < nv) d4[i] = step(a4[i], b4[i]);
         done = nv * 2;
     }
+    pdl_trigger();
     for (size_t i = done + tid; i < n; i += stride) d[i] = spec_binary_op<OP>(a[i], b[i]);
 }
 
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(kThreads) spec_mag_kernel(const float2 *a, flo
                                                            unsigned long long *keys) {
     __shared__ unsigned long long red[2 * (kThreads / 32)];
     unsigned long long kmin = 0, kmax = 0;
-    pdl_enter();
+    pdl_wait();
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     size_t done = 0;
@@ -146,6 +147,7 @@ __global__ void __launch_bounds__(kThreads) spec_mag_kernel(const float2 *a, flo
         if (i < nv) step(i, a4[2 * i], a4[2 * i + 1]);
         done = nv * 4;
     }
+    pdl_trigger();
     for (size_t i = done + tid; i < n; i += stride) {
         const float v = mag_op<LOG>(a[i], offset);
         d[i] = v;
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(kThreads) minmax_kernel(const float *x, size_t
                                                           unsigned long long *keys) {
     __shared__ unsigned long long red[2 * (kThreads / 32)];
     MinMaxRun run;
-    if constexpr (PARTIAL) pdl_enter();
+    if constexpr (PARTIAL) pdl_wait();
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     size_t done = 0;
@@ -237,6 +239,7 @@ __global__ void __launch_bounds__(kThreads) minmax_kernel(const float *x, size_t
         }
         done = nv * 4;
     }
+    if constexpr (PARTIAL) pdl_trigger();
     for (size_t i = done + tid; i < n; i += stride) run.add(x[i], (unsigned)i);
     if constexpr (PARTIAL) {
         const ulonglong2 k = block_minmax(min_key(run.vmin, run.imin), max_key(run.vmax, run.imax), red);
@@ -273,9 +276,9 @@ __global__ void __launch_bounds__(kThreads) normalize_kernel(const float *x, flo
         for (int k = 0; k < kBatch; k++)
             v[k] = i + k * stride < nv ? x4[i + k * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
     };
-    if constexpr (RAW) pdl_enter();
+    if constexpr (RAW) pdl_wait();
     fetch(tid);
-    if constexpr (!RAW) pdl_enter();
+    if constexpr (!RAW) pdl_wait();
     unsigned long long kmin = 0, kmax = 0;
     for (int i = threadIdx.x; i < parts; i += kThreads) {
         const ulonglong2 k = __ldcg(reinterpret_cast<const ulonglong2 *>(keys) + i);
@@ -296,6 +299,7 @@ __global__ void __launch_bounds__(kThreads) normalize_kernel(const float *x, flo
         s_lin = make_float2(f, (float)__dsub_rn(alpha, __dmul_rn((double)f, mn)));
     }
     __syncthreads();
+    pdl_trigger();
     const float scl = s_lin.x, c = s_lin.y;
     auto step = [&](const float4 q) {
         return make_float4(__fadd_rn(c, __fmul_rn(scl, q.x)), __fadd_rn(c, __fmul_rn(scl, q.y)),
