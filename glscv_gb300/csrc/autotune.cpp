@@ -102,11 +102,7 @@ int glsfft_set_fft_schedule(glsfft_context ctx, int rows, int cols, int row_sche
     if (!glsfft_schedule_available(cols, row_schedule, 0) ||
         !glsfft_schedule_available(rows, col_schedule, 1))
         return GLSFFT_ERROR_INVALID_VALUE;
-    const FftSchedule d = default_schedule(rows, cols);
-    if (row_schedule == d.row && col_schedule == d.col)
-        ctx->sched.erase(sched_key(rows, cols));
-    else
-        ctx->sched[sched_key(rows, cols)] = FftSchedule{row_schedule, col_schedule};
+    keep_schedule(ctx->sched, rows, cols, FftSchedule{row_schedule, col_schedule});
     return GLSFFT_SUCCESS;
 }
 
@@ -142,8 +138,7 @@ int glsfft_autotune_fft2d(glsfft_context ctx, int rows, int cols, int count,
         const int r = std::atoi(hit["row_schedule"].c_str());
         const int c = std::atoi(hit["col_schedule"].c_str());
         if (glsfft_schedule_available(cols, r, 0) && glsfft_schedule_available(rows, c, 1)) {
-            st = glsfft_set_fft_schedule(ctx, rows, cols, r, c);
-            if (st) return st;
+            keep_schedule(ctx->sched, rows, cols, FftSchedule{r, c}, count);
             res[0] = r;
             res[1] = c;
             res[2] = 1;
@@ -174,7 +169,7 @@ int glsfft_autotune_fft2d(glsfft_context ctx, int rows, int cols, int count,
     a.spread = 1;
     // each pass: its default schedule first, then the others in order; the
     // fastest is kept unless the default is within kKeepMargin of it
-    const FftSchedule dflt = default_schedule(rows, cols);
+    const FftSchedule dflt = default_schedule(rows, cols, count);
     for (int along_cols = 0; along_cols < 2 && !st; along_cols++) {
         const int n = along_cols ? rows : cols;
         const int first = along_cols ? dflt.col : dflt.row;
@@ -222,8 +217,7 @@ int glsfft_autotune_fft2d(glsfft_context ctx, int rows, int cols, int count,
         cudaGetLastError();
     }
     if (st) return st;
-    st = glsfft_set_fft_schedule(ctx, rows, cols, res[0], res[1]);
-    if (st) return st;
+    keep_schedule(ctx->sched, rows, cols, FftSchedule{res[0], res[1]}, count);
     if (cache_path && *cache_path) {
         key.push_back({"row_schedule", num(res[0])});
         key.push_back({"col_schedule", num(res[1])});

@@ -136,7 +136,8 @@ int grid_for(int device, int variant) {
 //     Not 1024-row images with a column-tiled workspace beyond 24 Mpx (64 x
 //     1024^2 there and back 602 / 608, 512 x 1024x128 592 / 578) or of fewer
 //     than 256 columns (384 x 1024x64 265 / 260, 56 x 1024x128 75 / 73), nor
-//     shorter images of 2048 columns beyond 24 Mpx (50 x 512x2048 480 / 472).
+//     shorter images of 2048 columns beyond 24 Mpx: 50 x 512x2048 480 / 472 while
+//     all their rows ran the schedule of small launches, 451 / 471 since.
 //     Over 338 runs of 15 sizes, 0.4 .. 50 Mpx, the launches came out 1.20
 //     times as fast as the persistent kernel.
 //   * images of the one-launch FFT gain at any total (4000 x 64^2 forward 63.6
@@ -213,8 +214,8 @@ std::vector<glsfft_batch_s::Segment> direct_segments(const std::vector<BatchImag
 bool use_direct(glsfft_batch plan) {
     if (plan->segments.empty() || plan->pinned || plan->args.stats) return false;
     for (const auto &sg : plan->segments) {
-        const FftSchedule sc = schedule_for(plan->ctx->sched, sg.rows, sg.cols),
-                          d = default_schedule(sg.rows, sg.cols);
+        const FftSchedule sc = schedule_for(plan->ctx->sched, sg.rows, sg.cols, sg.count),
+                          d = default_schedule(sg.rows, sg.cols, sg.count);
         if (sc.row != d.row || sc.col != d.col) return false;
     }
     return true;

@@ -222,7 +222,7 @@ int glsfft::fft2d_launch(glsfft_context ctx, const void *src, void *dst, int row
     const size_t px = (size_t)rows * cols;
     if (!src_step) src_step = px * (real_in ? sizeof(float) : sizeof(float2));
     if (!dst_step) dst_step = px * sizeof(float2);
-    const FftSchedule sc = schedule_for(ctx->sched, rows, cols);
+    const FftSchedule sc = schedule_for(ctx->sched, rows, cols, count);
     if (sc.row == 0 && sc.col == 0 && fused_applies(rows, cols)) {
         PassArgs a{};
         a.in0 = src;
@@ -555,7 +555,7 @@ static int one_pass(glsfft_context ctx, const void *src, void *dst, int count, i
     a.stall_ns = ctx->stall_ns;
     a.spread = 1;
     a.in_img_bytes = a.out_img_bytes = (size_t)rows * cols * sizeof(float2);
-    const FftSchedule sc = schedule_for(ctx->sched, rows, cols);
+    const FftSchedule sc = schedule_for(ctx->sched, rows, cols, count);
     cudaError_t e = along_rows ? launch_rows_sched(n, sc.row, a, count, s)
                                : launch_cols_sched(n, sc.col, a, count, s);
     return cuda_status(e);

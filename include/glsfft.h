@@ -204,7 +204,7 @@ GLSFFT_API int glsfft_schedule_available(int length, int schedule, int along_col
  * pass entry points and batch plans' own-launch images use for complex
  * rows x cols images on this context.  Until set or tuned, a size runs its
  * built-in default, measured on GB300: row schedule 2 for 2048- and
- * 4096-point rows (3 for up to 1024 of 2048 points), the streamed column pass for 4096-point columns,
+ * 4096-point rows (3 for up to 1024 of 2048 points in one launch), the streamed column pass for 4096-point columns,
  * schedule 0 otherwise; images of 16 points a side and more and at most 4096
  * pixels run both passes of fft2d / fft2d_batched in one launch (bit-identical
  * to schedules 0, 0) until another pair is set. */
