@@ -241,6 +241,14 @@ void dispatcher_main(glsfft_server srv) {
             const Request snapshot = rq;
             lock.unlock();
             const int st = launch_request(srv, ref, snapshot, slot);
+            if (st != GLSFFT_SUCCESS) {
+                // what was issued before the failure still uses the frame and
+                // the workspace: the copy kernel on the link stream, the rest
+                // on the slot's
+                if (snapshot.linked) cudaStreamSynchronize(srv->link);
+                cudaStreamSynchronize(slot.stream);
+                cudaGetLastError();
+            }
             lock.lock();
             if (st != GLSFFT_SUCCESS) {
                 Request &r2 = srv->reqs[ticket];
