@@ -692,8 +692,9 @@ int glsfft_batch_autotune(glsfft_batch plan, const char *cache_path, int reps, v
         return st;
     }
 
-    // 2. the plan key: device, the persistent images' and the other images'
-    //    size histograms, the transform flags
+    // 2. the plan key: device, whether the default schedule is pass launches
+    //    (it depends on where the images lie), the persistent images' and the
+    //    other images' size histograms, the transform flags
     auto histogram = [](const std::map<std::pair<int, int>, int> &h) {
         std::string o;
         for (const auto &kv : h) {
@@ -708,7 +709,7 @@ int glsfft_batch_autotune(glsfft_batch plan, const char *cache_path, int reps, v
     std::string flags;
     for (int f : plan->flags) flags += (flags.empty() ? "" : ",") + std::to_string(f);
     plan_cache::Pairs key = device_fields(plan->device);
-    key.push_back({"kind", plan_cache::quote("batch")});
+    key.push_back({"kind", plan_cache::quote(plan->segments.empty() ? "batch" : "batch_runs")});
     key.push_back({"persistent", plan_cache::quote(histogram(pers))});
     key.push_back({"others", plan_cache::quote(histogram(other_sizes))});
     key.push_back({"flags", plan_cache::quote(flags)});

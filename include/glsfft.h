@@ -415,7 +415,7 @@ GLSFFT_API int glsfft_batch_get_schedule(glsfft_batch plan, int *schedule4);
  * unless the default schedule is within 1% of it.  With cache_path
  * set, the choice is looked up in / appended to that plan cache file
  * (keyed by device, driver, library version, the plan's size histograms and
- * flags); a hit is applied without timing.
+ * flags, and whether its images lie in runs that pass launches take); a hit is applied without timing.
  * result[6] = {variant, claim_chunk, claim_ahead, lag_items, 1 if from the
  * cache, candidates timed}; ms[2] = {chosen, default} per execution.
  * Either may be NULL.
