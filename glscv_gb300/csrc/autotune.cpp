@@ -198,13 +198,12 @@ int glsfft_autotune_fft2d(glsfft_context ctx, int rows, int cols, int count,
         t[1] += base;
     }
     if (!st && fused_applies(rows, cols)) {
-        // the default of these sizes is one launch for both passes: it stays
-        // unless two passes are faster by the margin
+        // the default of these sizes is one launch for both passes
         double m = 0.0;
         st = time_median_ms([&]() { return cuda_status(launch_fused(a, false, 1.0f, count, s)); }, 2, 7,
                             s, &m);
         t[1] = m;
-        if (t[0] >= m * (1.0 - kKeepMargin)) {
+        if (one_launch_stays(m, t[0], FftSchedule{res[0], res[1]}, dflt, kKeepMargin)) {
             t[0] = m;
             res[0] = dflt.row;
             res[1] = dflt.col;

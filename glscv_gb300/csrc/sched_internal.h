@@ -38,6 +38,14 @@ inline FftSchedule schedule_for(const Map &m, int rows, int cols, int images = 1
     const auto it = m.find(sched_key(rows, cols));
     return it != m.end() ? it->second : default_schedule(rows, cols, images);
 }
+// Sizes that run both passes in one launch by default: whether that stays when
+// the tuner's best pair of passes `two` took two_ms and the one launch one_ms.
+// It does unless the pair is faster by `margin`, and when the pair is the
+// default one, which cannot be asked for apart from it.
+inline bool one_launch_stays(double one_ms, double two_ms, FftSchedule two, FftSchedule dflt,
+                             double margin) {
+    return two_ms >= one_ms * (1.0 - margin) || (two.row == dflt.row && two.col == dflt.col);
+}
 // Keep `s`, chosen for `images` images, for a size: the built-in choice needs
 // no entry, but a choice that differs for one image is kept as made.
 template <class Map>

@@ -40,6 +40,13 @@ int main() {
         keep_schedule(m, 512, 2048, FftSchedule{row, 0}, 50);
         CHECK(schedule_for(m, 512, 2048).row == row && schedule_for(m, 512, 2048, 50).row == row);
     }
+    // one launch for both passes: a pair of passes must beat it by the margin
+    // and be one that runs when it is set
+    const FftSchedule d = default_schedule(64, 64), other{1, 0};
+    CHECK(one_launch_stays(1.0, 1.5, other, d, 0.01) && one_launch_stays(1.0, 0.995, other, d, 0.01));
+    CHECK(!one_launch_stays(1.0, 0.9, other, d, 0.01));
+    CHECK(one_launch_stays(1.0, 0.9, d, d, 0.01));
+
     std::printf(failures ? "%d FAILED\n" : "ALL OK\n", failures);
     return failures != 0;
 }
