@@ -79,6 +79,7 @@ _SIGNATURES = {
     "glsfft_batch_status": (_ip, [_vp, _vp]),
     "glsfft_batch_info": (_ip, [_vp, ctypes.POINTER(_ip), ctypes.POINTER(_ip),
                                 ctypes.POINTER(_ip)]),
+    "glsfft_batch_uses_launches": (_ip, [_vp, ctypes.POINTER(_ip)]),
     "glsfft_batch_workspace": (_ip, [_vp, ctypes.POINTER(_ip), ctypes.POINTER(_sz)]),
     "glsfft_batch_inject_stall": (_ip, [_vp, ctypes.c_longlong]),
     "glsfft_batch_get_schedule": (_ip, [_vp, ctypes.POINTER(_ip)]),
@@ -351,6 +352,12 @@ class Batch:
         check(lib().glsfft_batch_info(self.handle, ctypes.byref(a), ctypes.byref(b),
                                       ctypes.byref(c)), "batch_info")
         return {"persistent_images": a.value, "items": b.value, "grid": c.value}
+
+    def uses_launches(self) -> bool:
+        """Whether batched pass launches run in place of the persistent kernel."""
+        n = _ip()
+        check(lib().glsfft_batch_uses_launches(self.handle, ctypes.byref(n)), "batch_uses_launches")
+        return bool(n.value)
 
     def workspace(self):
         """glsfft_batch_workspace: images with a column-tiled workspace and

@@ -619,6 +619,12 @@ int glsfft_batch_info(glsfft_batch plan, int *persistent_images, int *items, int
     return GLSFFT_SUCCESS;
 }
 
+int glsfft_batch_uses_launches(glsfft_batch plan, int *launches) {
+    if (!plan || !launches) return GLSFFT_ERROR_INVALID_VALUE;
+    *launches = plan->direct ? 1 : 0;
+    return GLSFFT_SUCCESS;
+}
+
 int glsfft_batch_workspace(glsfft_batch plan, int *tiled_images, size_t *bytes) {
     if (!plan) return GLSFFT_ERROR_INVALID_VALUE;
     int n = 0;

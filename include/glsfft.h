@@ -377,6 +377,10 @@ GLSFFT_API int glsfft_batch_status(glsfft_batch plan, void *stream);
 GLSFFT_API int glsfft_batch_info(glsfft_batch plan, int *persistent_images, int *items,
                                  int *grid);
 
+/* *launches: 1 while the plan's graph holds batched pass launches in place of
+ * the persistent one (glsfft_batch_create), else 0. */
+GLSFFT_API int glsfft_batch_uses_launches(glsfft_batch plan, int *launches);
+
 /*
  * The plan's column-tiled workspace: images of the persistent launch with
  * 1024 rows and 16 <= cols <= 1024 get one image-sized device buffer each
