@@ -93,7 +93,8 @@ struct PassArgs {
     // for it, so the wait runs out
     long long stall_ns;
     // a small grid may take other block shapes, to spread evenly over the SMs
-    // (row_lines, cols_t): not a launch beside other streams' (the server's)
+    // (row_lines, cols_t), and lets its successor in late (launch_pass): not a
+    // launch that always runs beside other streams' (the server's)
     int spread;
     // launch with programmatic dependent launch (every pass kernel begins
     // with griddepcontrol.wait): the grid may become resident before its
