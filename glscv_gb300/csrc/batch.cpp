@@ -119,32 +119,32 @@ int grid_for(int device, int variant) {
 // the passes find the images in L2.  Measured on GB300, us per execution,
 // launches against the persistent kernel:
 //   * up to 64 MiB of images (128 MiB with their sources; 48 MiB there and
-//     back), at most eight runs, each a launch per pass on a graph branch of its own: 2 x 256x512 forward
-//     8.2 / 17.7, 16 x 256^2 12.4 / 18.6, 8 x 512^2 16.5 / 27.4; 8 x 1024^2
-//     49.3 / 52.5 in one run, 45.7 in eight; eight mixed sizes 18.2 .. 33.8 /
+//     back), at most eight runs, each a launch per pass on a graph branch of its
+//     own: 2 x 256x512 forward 6.5 / 17.4, 16 x 256^2 10.5 / 16.9, 8 x 512^2
+//     14.6 / 24.9; 8 x 1024^2 47.4 / 52.3; eight mixed sizes 18.2 .. 33.8 /
 //     20.8 .. 35.1, there and back 30.7 .. 60.6 / 35.4 .. 62.2; with twelve the
 //     launches themselves take as long as the persistent kernel (39 / 38).
-//   * one larger run in pieces of about 3 Mpx (24 MiB; at most 3.5, an even
-//     number of them: 14 Mpx there and back 2 .. 7 % faster in four pieces than
-//     in six, 7 Mpx 10 .. 15 % in two than in four), each through all its passes
-//     before the next, on two branches, so that the pieces in flight stay in
-//     L2: 24 x 1024^2 120 / 133, there and back 230 / 243; 96 x 512^2
-//     114 / 124 and 216 / 233; 384 x 256^2 93 / 107 and 165 / 186; 1024 x 256^2
-//     237 / 266 and 428 / 474; 12 x 1024x2048 132 / 143 and 250 / 270.  As one
-//     launch per pass 24 x 1024^2 took 142 and 280; pieces of 2 or 4 Mpx or
-//     more branches are up to 10 % slower.
-//     Not 1024-row images with a column-tiled workspace beyond 24 Mpx (64 x
-//     1024^2 there and back 602 / 608, 512 x 1024x128 592 / 578) or of fewer
-//     than 256 columns (384 x 1024x64 265 / 260, 56 x 1024x128 75 / 73), nor
-//     shorter images of 2048 columns beyond 24 Mpx: 50 x 512x2048 480 / 472 while
-//     all their rows ran the schedule of small launches, 451 / 471 since.
-//     Over 338 runs of 15 sizes, 0.4 .. 50 Mpx, the launches came out 1.20
-//     times as fast as the persistent kernel.
-//   * images of the one-launch FFT gain at any total (4000 x 64^2 forward 63.6
-//     / 86.2, there and back 123 / 157);
+//   * one larger run in pieces of about 3 Mpx (24 MiB): 2 ceil(size / 7 Mpx)
+//     pieces, as equal as whole images come, or one per image where there are
+//     fewer (14 Mpx there and back 2 .. 7 % faster in four pieces than in six, 7
+//     Mpx 10 .. 15 % in two than in four), each through all its passes before the next, on two
+//     branches, so that the pieces in flight stay in L2: 24 x 1024^2 120 / 131,
+//     there and back 228 / 242; 96 x 512^2 113 / 123 and 215 / 231; 1024 x 256^2
+//     239 / 264 and 427 / 472; 12 x 1024x2048 127 / 141 and 240 / 268; 25 x
+//     1024x2048 255 / 282 and 490 / 550.  As one launch per pass 24 x 1024^2
+//     took 142 and 280; pieces of 2 or 4 Mpx or more branches are up to 10 %
+//     slower.
+//     Not 1024-row images of fewer than 256 columns with a column-tiled
+//     workspace (384 x 1024x64 265 / 260, 56 x 1024x128 75 / 73), which beyond
+//     24 Mpx lose more (512 x 1024x128 there and back 592 / 578).  Beyond 24 Mpx
+//     wider 1024-row images and shorter ones of 2048 columns stay out too, on
+//     older times; they would gain now (there and back 64 x 1024^2 600 / 606, 96 x
+//     1024x512 455 / 471, 50 x 512x2048 451 / 471).
+//   * images of the one-launch FFT gain at any total (4000 x 64^2 forward 61.2
+//     / 84.3, there and back 120 / 154);
 //   * images of 32 columns up to 16 MiB, of 16 up to 4, whose rows the pass
-//     kernels read in short pieces: 64 x 512x32 there and back 1.25 times as
-//     fast, 256 x 512x32 1.05, 505 x 512x32 0.96; 64 x 512x16 1.56, 128 x
+//     kernels read in short pieces: 64 x 512x32 there and back 31.0 / 40.4, 256 x
+//     512x32 1.05 times as fast, 505 x 512x32 0.96; 64 x 512x16 31.0 / 41.6, 128 x
 //     512x16 0.94.
 constexpr size_t direct_bytes(size_t transforms) { return size_t(transforms > 1 ? 48 : 64) << 20; }
 constexpr size_t kNarrowBytes = size_t(4) << 20;

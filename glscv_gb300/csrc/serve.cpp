@@ -87,8 +87,8 @@ constexpr int kDispatchers = 3;
 // reads a large frame itself holds the registers of every SM for as long as
 // the link takes, and the others' column kernels wait.  Smaller frames, and a
 // request on its own, are sooner done without the extra launch and event.
-// GB300, bursts of six, read by the row kernel / copied: 2048^2 831 / 640 us,
-// 1024^2 236 / 213, 512^2 133 / 139; alone 2048^2 189 / 190.
+// GB300, bursts of six, read by the row kernel / copied: 2048^2 772 / 600 us,
+// 1024^2 224 / 203, 512^2 130 / 136.
 constexpr size_t kLinkedPixels = (size_t)1 << 20;
 
 size_t workspace_bytes(int rows, int cols) {

@@ -191,8 +191,8 @@ __global__ void minmax_reset_kernel(unsigned long long *keys) {
 constexpr int kMinMaxBatch = 8;
 // Its blocks: enough for every thread to fill one batch, or two per SM while
 // that is fewer (a thread runs its whole batch, so a grid of one load per
-// thread spent seven of eight slots on nothing: 1081 x 1919 with
-// normalisation 10.2 us, 7.0 with this).
+// thread spends seven of eight slots on nothing: 1081 x 1919 with
+// normalisation 10.1 us, 6.7 with this).
 template <bool PARTIAL>
 int minmax_grid(size_t n);
 
@@ -291,8 +291,8 @@ __global__ void __launch_bounds__(kThreads) normalize_kernel(const float *x, flo
         kmax = k.y;
     }
     // one thread runs the FP64 steps: GB300's FP64 pipe takes 16 cycles a
-    // warp instruction, and every thread computing them cost the pass about
-    // 4 us (1081 x 1919: min / max and normalisation 11.2 -> 5.6 us)
+    // warp instruction (1081 x 1919, min / max and normalisation: 8.0 us with
+    // every thread computing them, 6.7 with one)
     if (threadIdx.x == 0) {
         const double mn = min_key_value(kmin), mx = max_key_value(kmax);
         const float f = __fdiv_rn((float)(beta - alpha), (float)(mx - mn));
@@ -474,7 +474,11 @@ int glsfft_normalize_minmax(glsfft_context ctx, const float *src, float *dst, in
     // reduce them (a reset and atomics would be a third)
     const int parts = std::min(minmax_grid<true>(n), ctx->key_pairs);
     unsigned long long *keys = nullptr;
-    st = keys_at(ctx, 0, &keys);  // the workspace is used, as ever
+    // the blocks' keys have memory of their own (d_keys), but the call keeps
+    // its contract: it claims the workspace like the other reductions, so it
+    // ends the last phaseCorrelate's surface and fails where the budget has no
+    // room for them
+    st = keys_at(ctx, 0, &keys);
     if (st) return st;
     keys = ctx->d_keys;
     cudaStream_t s = (cudaStream_t)stream;
